@@ -251,12 +251,11 @@ struct BsdfSample
 	bool  ok;
 };
 
-// bsdf_eval / bsdf_pdf / bsdf_sample are kept out of line: each holds all three surface optics,
-// and the shade kernel calls pdf twice. Inlined copies made that kernel large enough to stall
-// on instruction fetch.
+// Inlined: the shading kernels are instantiated per material type and fix mat.type before they
+// call these, so that each copy keeps one surface optics only.
 //
 // calcBsdf: returns false when not measurable.
-static __device__ __noinline__ bool bsdf_eval(const Material& mat, const Frame& f, V3 l, V3 v, RGB* out)
+__device__ __forceinline__ bool bsdf_eval(const Material& mat, const Frame& f, V3 l, V3 v, RGB* out)
 {
 	if(!sidedness_agreed(f, l) || !sidedness_agreed(f, v) || mat.type == PG_MAT_ABSORBER)
 	{
@@ -350,7 +349,7 @@ static __device__ __noinline__ bool bsdf_eval(const Material& mat, const Frame& 
 
 // calcBsdfPdf: returns the solid-angle pdf, or 0 for an empty/invalid pdf (the reference's
 // `operator bool` on lta::PDF requires a finite positive value).
-static __device__ __noinline__ float bsdf_pdf(const Material& mat, const Frame& f, V3 l, V3 v)
+__device__ __forceinline__ float bsdf_pdf(const Material& mat, const Frame& f, V3 l, V3 v)
 {
 	if(!sidedness_agreed(f, l) || !sidedness_agreed(f, v) || mat.type == PG_MAT_ABSORBER)
 	{
@@ -428,7 +427,7 @@ static __device__ __noinline__ float bsdf_pdf(const Material& mat, const Frame& 
 
 // genBsdfSample with three uniform numbers (u0, u1 for the direction, u2 for the dielectric
 // reflect/transmit pick, which the reference draws with `unflowedPick`).
-static __device__ __noinline__ BsdfSample bsdf_sample(const Material& mat, const Frame& f, V3 v, float u0, float u1, float u2)
+__device__ __forceinline__ BsdfSample bsdf_sample(const Material& mat, const Frame& f, V3 v, float u0, float u1, float u2)
 {
 	BsdfSample s;
 	s.ok = false;

@@ -29,6 +29,11 @@ namespace
 {
 
 constexpr int kShadeBlock = 128;
+// Blocks per SM the shading kernels are compiled for (64 registers). They are bound by the latency of
+// their dependent loads and of long FP32 chains, so a full SM is worth the few spilled words: shading
+// and refinery of the bench scene at 16 samples 5.57 ms at 4 blocks (80 to 92 registers, no
+// spills), 5.66 ms at 6, 4.98 ms at 8; of the quarter-scale city 9.70, 10.06 and 8.74 ms.
+constexpr int kShadeMinBlocks = 8;
 // Iterations per training period of a guided render that trains (even: the path buffers alternate).
 // Periods of 6 and 8 iterations measured the same equal-time ratio on the slit room within the
 // run-to-run spread, with fewer training steps.
@@ -250,10 +255,16 @@ __device__ __forceinline__ bool guided_vertex(const Material& m, uint32_t meta, 
 	return !(meta & kMetaStopAfter) && (meta & kMetaBounceMask) < guide_depth && guidable(m);
 }
 
-// Lists every slot of the current queue under its shading class (kShadeClasses): 0 for a miss,
-// 1 + the material type of the hit surface, or kGuidedClass for a vertex a guided render guides
-// (guide_depth > 0: the vertices below that bounce), in the list of that class for this block's
-// residue (kClassLists). Lanes of one class share one atomic. `list_capacity` bounds the slots one
+__device__ __forceinline__ uint32_t class_of(uint32_t material_type)
+{
+	return material_type == PG_MAT_MATTE ? kClassMatte
+	       : material_type == PG_MAT_CONDUCTOR ? kClassConductor
+	       : material_type == PG_MAT_DIELECTRIC ? kClassDielectric : kClassAbsorber;
+}
+
+// Lists every slot of the current queue under its shading class (ShadeClass; kClassGuided for a
+// vertex a guided render guides -- guide_depth > 0: the vertices below that bounce), in the list of
+// that class for this block's residue (kClassLists). Lanes of one class share one atomic. `list_capacity` bounds the slots one
 // list can receive: the slots all blocks of one residue visit in the grid-stride loop.
 // MULTI: the hit triangle belongs to the scene in the top bits of the slot's meta word.
 template<bool MULTI>
@@ -267,19 +278,18 @@ classify_kernel(DeviceScene s_single, RenderCounters* __restrict__ c, const uint
 	for(uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
 	{
 		const uint32_t tri = hits[i].x;
-		uint32_t cls = 0u;
+		uint32_t cls = kClassMiss;
 		if(tri != 0xFFFFFFFFu)
 		{
 			if constexpr(MULTI)
 			{
 				const DeviceScene& s = batch.scenes[meta[i] >> kMetaSceneShift].scene;
-				cls = min(1u + s.materials[__ldg(&s.tris[tri].material)].type, kGuidedClass - 1u);
+				cls = class_of(s.materials[__ldg(&s.tris[tri].material)].type);
 			}
 			else
 			{
 				const Material& m = s_single.materials[__ldg(&s_single.tris[tri].material)];
-				cls = guide_depth > 0u && guided_vertex(m, meta[i], guide_depth) ? kGuidedClass
-				                                                                 : min(1u + m.type, kGuidedClass - 1u);
+				cls = guide_depth > 0u && guided_vertex(m, meta[i], guide_depth) ? kClassGuided : class_of(m.type);
 			}
 		}
 		const uint32_t list = cls * kClassLists + residue;
@@ -524,7 +534,7 @@ struct ShadeArgs
 	GuideArgs     guide;
 	RefineSettings refine;
 	RefineQueue   refine_queue;   // iterative refine mode: requests for refine_kernel
-	const uint32_t* order;        // slots listed per shading class (classify_kernel), or null: slot order
+	const uint32_t* order;        // slots listed per shading class (classify_kernel)
 	uint32_t      order_capacity; // slots per list of `order`
 	BatchView     batch;          // multi-scene renders: scene, film and numbering of every path
 };
@@ -532,39 +542,69 @@ struct ShadeArgs
 __device__ __forceinline__ float4 cur_gf0(const ShadeArgs& a, uint32_t i) { return a.cur.gf0[i]; }
 __device__ __forceinline__ float4 cur_gf1(const ShadeArgs& a, uint32_t i) { return a.cur.gf1[i]; }
 
+// The shading kernels, one per material kind: each takes the slots of its classes, and its code
+// and registers are those of one surface optics, inlined. (One kernel for all kinds called the optics
+// out of line, with the material and the frame passed through local memory, at 94 registers; the
+// bench scene's shading and refinery at 16 samples took 5.95 ms instead of 4.98 ms, the quarter-scale
+// city's 10.97 ms instead of 8.74 ms. Inlined into that one kernel, they made it stall on
+// instruction fetch.)
+enum ShadeKind : int
+{
+	kShadeMatte = 0,        // misses, light surfaces, matte and guided vertices
+	kShadeConductor = 1,
+	kShadeDielectric = 2,
+};
+
 // GUIDED instantiates the learned-guiding paths; the plain estimator compiles without them.
 // MULTI: each path shades in the scene of its meta word's top bits (a.batch), into that scene's
 // film, and passes the scene on to its continuation and its NEE record.
-template<bool GUIDED, bool MULTI>
-__global__ void __launch_bounds__(kShadeBlock)
+template<bool GUIDED, bool MULTI, int KIND>
+__global__ void __launch_bounds__(kShadeBlock, kShadeMinBlocks)
 shade_kernel(ShadeArgs a)
 {
-	const uint32_t total = a.counters->n_total;
-	// work item w -> queue slot: list by list (class-major) through the lists classify_kernel made
-	__shared__ uint32_t list_end[kOrderLists];
-	if(a.order && threadIdx.x == 0)
+	constexpr uint32_t kFirstList = (KIND == kShadeMatte ? kClassMiss
+	                                 : KIND == kShadeConductor ? kClassConductor : kClassDielectric) * kClassLists;
+	constexpr uint32_t kLists = (KIND == kShadeMatte ? 4u : 1u) * kClassLists;
+	// work item w -> queue slot: list by list (class-major) through the lists classify_kernel made.
+	// One warp sums up the list lengths (one thread loading them one after another took longer than
+	// shading a small queue).
+	__shared__ uint32_t list_end[kLists];
+	if(threadIdx.x < 32u)
 	{
-		uint32_t end = 0;
-		for(uint32_t l = 0; l < kOrderLists; ++l)
+		uint32_t before = 0;
+		#pragma unroll
+		for(uint32_t l0 = 0; l0 < kLists; l0 += 32u)
 		{
-			end += a.counters->n_class[l];
-			list_end[l] = end;
+			const uint32_t l = l0 + threadIdx.x;
+			uint32_t end = l < kLists ? a.counters->n_class[kFirstList + l] : 0u;
+			#pragma unroll
+			for(uint32_t d = 1; d < 32u; d *= 2u)
+			{
+				const uint32_t up = __shfl_up_sync(0xFFFFFFFFu, end, d);
+				end += threadIdx.x >= d ? up : 0u;
+			}
+			end += before;
+			if(l < kLists)
+			{
+				list_end[l] = end;
+			}
+			before = __shfl_sync(0xFFFFFFFFu, end, 31);
 		}
 	}
 	__syncthreads();
+	const uint32_t total = list_end[kLists - 1u];
 	for(uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < total; w += gridDim.x * blockDim.x)
 	{
-		uint32_t i = w;
-		if(a.order)
+		uint32_t i;
 		{
 			// first list whose end exceeds w
-			uint32_t lo = 0, hi = kOrderLists - 1u;
+			uint32_t lo = 0, hi = kLists - 1u;
 			while(lo < hi)
 			{
 				const uint32_t mid = (lo + hi) >> 1;
 				if(w < list_end[mid]) { hi = mid; } else { lo = mid + 1u; }
 			}
-			i = a.order[lo * a.order_capacity + (w - (lo ? list_end[lo - 1u] : 0u))];
+			i = a.order[(kFirstList + lo) * a.order_capacity + (w - (lo ? list_end[lo - 1u] : 0u))];
 		}
 		const uint32_t p = a.cur.path[i];
 		const uint32_t meta = a.cur.meta[i];
@@ -646,7 +686,7 @@ shade_kernel(ShadeArgs a)
 		};
 
 		// ---- miss: environment (the dome primitive is hit after every triangle missed)
-		if(hit.x == 0xFFFFFFFFu)
+		if(KIND == kShadeMatte && hit.x == 0xFFFFFFFFu)
 		{
 			const RGB le = s.env_emitter < 0 ? RGB{0.0f, 0.0f, 0.0f} : env_lookup(s.env_map, env_uv(s.env_map, d));
 			if(train_row != 0xFFFFFFFFu && s.env_emitter >= 0)
@@ -756,7 +796,9 @@ shade_kernel(ShadeArgs a)
 		{
 			rec_scale = train_wfac / fmaxf(luminance(throughput), 1e-20f);
 		}
-		const Material mat = s.materials[mat_index];
+		Material mat = s.materials[mat_index];
+		const bool absorber = KIND == kShadeMatte && mat.type == PG_MAT_ABSORBER;
+		mat.type = KIND == kShadeMatte ? PG_MAT_MATTE : KIND == kShadeConductor ? PG_MAT_CONDUCTOR : PG_MAT_DIELECTRIC;
 		const V3 v = -d;
 
 		// ---- next-event estimation (TDirectLightEstimator::neeSampleEmission,
@@ -771,15 +813,15 @@ shade_kernel(ShadeArgs a)
 		RGB sh_c{};
 		uint32_t nee_row = 0xFFFFFFFFu;   // this vertex's NEE direction as a training sample of its own
 		float nee_w = 0.0f;
-		const uint32_t grow = GUIDED ? a.guide.map[i] : 0xFFFFFFFFu;
-		const bool guided = GUIDED && grow != 0xFFFFFFFFu;
+		const uint32_t grow = GUIDED && KIND == kShadeMatte ? a.guide.map[i] : 0xFFFFFFFFu;
+		const bool guided = GUIDED && KIND == kShadeMatte && grow != 0xFFFFFFFFu;
 		const float* graw = guided ? a.guide.raw + static_cast<size_t>(grow) * guide::kMixFloats : nullptr;
 		const float alpha = a.guide.alpha;
 		// Every material here is non-delta, so NEE applies at every vertex of BNEEPT
 		// (TDirectLightEstimator::isNeeSamplable); a black Lambertian surface can gain nothing
 		// from it, so its shadow ray is skipped (its contribution would be exactly zero).
-		const bool black_matte = (mat.type == PG_MAT_MATTE && mat.cr == 0.0f && mat.cg == 0.0f && mat.cb == 0.0f) ||
-		                         mat.type == PG_MAT_ABSORBER;
+		const bool black_matte = KIND == kShadeMatte &&
+		                         ((mat.cr == 0.0f && mat.cg == 0.0f && mat.cb == 0.0f) || absorber);
 		const bool nee_samplable = !bvpt;
 		const bool use_nee = nee_samplable && s.num_emitters > 0 && !black_matte;
 		if(use_nee)
@@ -949,6 +991,10 @@ shade_kernel(ShadeArgs a)
 				}
 			}
 		}
+		else if(absorber)
+		{
+			bs.ok = false;
+		}
 		else
 		{
 			bs = bsdf_sample(mat, frame, v, rng.u01(bounce, DIM_BSDF_0),
@@ -1070,6 +1116,23 @@ shade_kernel(ShadeArgs a)
 			}
 		}
 	}
+}
+
+// The shading launches of one iteration: the matte kernel (which also ends misses), and the kernels
+// of the other kinds that the scene's materials have (bit KIND of `kinds`).
+template<bool GUIDED, bool MULTI>
+void launch_shade(const ShadeArgs& sa, uint32_t kinds, int grid, cudaStream_t st)
+{
+	shade_kernel<GUIDED, MULTI, kShadeMatte><<<grid, kShadeBlock, 0, st>>>(sa);
+	if(kinds & (1u << kShadeConductor))
+	{
+		shade_kernel<GUIDED, MULTI, kShadeConductor><<<grid, kShadeBlock, 0, st>>>(sa);
+	}
+	if(kinds & (1u << kShadeDielectric))
+	{
+		shade_kernel<GUIDED, MULTI, kShadeDielectric><<<grid, kShadeBlock, 0, st>>>(sa);
+	}
+	PG_CUDA_CHECK(cudaGetLastError());
 }
 
 // The surface refinery of one iteration (iterative refine mode): every queued ray slot holds the
@@ -1222,6 +1285,8 @@ RenderScene::RenderScene(const SceneDesc& desc, float max_origin_abs)
 	for(const Material& m : desc.materials)
 	{
 		m_material_types.push_back(m.type);
+		m_shade_kinds |= m.type == PG_MAT_CONDUCTOR ? 1u << kShadeConductor
+		                 : m.type == PG_MAT_DIELECTRIC ? 1u << kShadeDielectric : 0u;
 	}
 
 	// scene bound, normalising the guiding network's position inputs
@@ -1991,6 +2056,7 @@ float RenderScene::render_batch(const std::vector<const RenderScene*>& scenes, c
 			b.first_global = sample * wh;
 			b.width_height = static_cast<uint32_t>(wh);
 			b.spp = take;
+			b.shade_kinds = sc.m_shade_kinds;
 			chunk.push_back(b);
 			acc += wh * take;
 			sample += take;
@@ -2176,6 +2242,16 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 		PG_CUDA_CHECK(cudaMemsetAsync(m_gscalars.get(), 0, 4 * sizeof(float), st));
 	}
 	RenderCounters* const d_counters = m_counters.get();
+	// the shading kernels this render's materials need
+	uint32_t kinds = m_shade_kinds;
+	if(multi)
+	{
+		kinds = 0;
+		for(const BatchScene& b : *batch)
+		{
+			kinds |= b.shade_kinds;
+		}
+	}
 	// The NEE segments made by an iteration's shading are traced by the next iteration's
 	// trace_kernel together with its closest-hit rays (one launch, one tail). Training runs in
 	// periods of P = kTrainPeriod iterations (position q = iteration mod P):
@@ -2265,17 +2341,16 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 		sa.batch = bview;
 		if(multi)
 		{
-			shade_kernel<false, true><<<grid, kShadeBlock, 0, st>>>(sa);
+			launch_shade<false, true>(sa, kinds, grid, st);
 		}
 		else if(guided)
 		{
-			shade_kernel<true, false><<<grid, kShadeBlock, 0, st>>>(sa);
+			launch_shade<true, false>(sa, kinds, grid, st);
 		}
 		else
 		{
-			shade_kernel<false, false><<<grid, kShadeBlock, 0, st>>>(sa);
+			launch_shade<false, false>(sa, kinds, grid, st);
 		}
-		PG_CUDA_CHECK(cudaGetLastError());
 		if(params.refine_mode == PG_REFINE_ITERATIVE)
 		{
 			if(multi)
@@ -2392,7 +2467,7 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 			iteration(q, nullptr);
 		}
 		PG_CUDA_CHECK(cudaStreamEndCapture(st, &graph));
-		const int key = (guided ? 1 : 0) | (training ? 2 : 0) | (multi ? 4 : 0);
+		const int key = (guided ? 1 : 0) | (training ? 2 : 0) | (multi ? 4 : 0) | static_cast<int>(kinds << 3);
 		bool updated = false;
 		if(m_exec && m_exec_key == key)
 		{
@@ -2492,10 +2567,10 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 	m_last_shadow = final_counters.shadow_rays;
 	m_last_iterations = iterations;
 	{
-		// prepare, regen, trace + classify (or extend + shadow), shade (+ refine in the iterative
+		// prepare, regen, trace + classify, shade per material kind (+ refine in the iterative
 		// mode); guide query + forward; training: weight sums (and clamp), forward, backward, Adam,
 		// step, repack, loss
-		const unsigned long long per_iteration = 5ull +
+		const unsigned long long per_iteration = 5ull + ((kinds >> kShadeConductor) & 1u) + ((kinds >> kShadeDielectric) & 1u) +
 		                                         (params.refine_mode == PG_REFINE_ITERATIVE ? 1ull : 0ull) +
 		                                         (guided ? 2ull : 0ull);
 		const unsigned long long per_step = training ? (m_guide_params.clamp > 0.0f ? 8ull : 6ull) : 0ull;

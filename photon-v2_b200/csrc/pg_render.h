@@ -181,15 +181,22 @@ struct DeviceScene
 	Camera            cam;
 };
 
-// Shading classes of a closest-hit result: 0 = miss, then 1 + the hit surface's material type
-// (matte, conductor, dielectric, absorber), and last the matte vertices that a guided render
-// guides (kGuidedClass), whose shading also evaluates and samples the learned mixture: kept apart,
-// they fill whole warps instead of making every matte warp wait on its guided lanes.
-// classify_kernel lists the queue slots of each class so that the shading kernel's warps mostly
-// run one code path. Each class has kClassLists lists, one per residue of the block index, so that
-// the list counters' atomics spread over kOrderLists addresses instead of queuing on six.
+// Shading classes of a closest-hit result. classify_kernel lists the queue slots of each class, and
+// each shading kernel takes the classes of its material kind: the matte kernel the first four (a
+// guided vertex also evaluates and samples the learned mixture: in a class of its own it fills whole
+// warps instead of making every matte warp wait on its guided lanes), the conductor and the
+// dielectric kernel one each. Each class has kClassLists lists, one per residue of the block index,
+// so that the list counters' atomics spread over kOrderLists addresses instead of queuing on six.
+enum ShadeClass : uint32_t
+{
+	kClassMiss = 0,
+	kClassAbsorber = 1,     // the surface of an area light: its emission ends the path
+	kClassMatte = 2,
+	kClassGuided = 3,       // a matte vertex that a guided render guides
+	kClassConductor = 4,
+	kClassDielectric = 5,
+};
 constexpr uint32_t kShadeClasses = 6;
-constexpr uint32_t kGuidedClass = kShadeClasses - 1u;
 constexpr uint32_t kClassLists = 16;
 constexpr uint32_t kOrderLists = kShadeClasses * kClassLists;
 
@@ -271,6 +278,7 @@ struct BatchScene
 	unsigned long long first_global;
 	uint32_t    width_height;
 	uint32_t    spp;
+	uint32_t    shade_kinds;   // RenderScene::m_shade_kinds of the scene
 };
 
 // The scene table of a multi-scene render (device memory).
@@ -422,6 +430,7 @@ private:
 	float m_max_origin_abs = 0.0f;
 	uint32_t m_bvh_builder = 0;
 	std::vector<uint32_t> m_material_types;   // per material (fingerprint)
+	uint32_t m_shade_kinds = 0;               // bit per shading kernel the materials need besides the matte one
 	DeviceBuffer<uint32_t> m_path[2], m_meta[2];
 	DeviceBuffer<float4>   m_thr[2], m_rad[2], m_prev[2], m_ro[2], m_rd[2];
 	DeviceBuffer<uint2>    m_hits;
