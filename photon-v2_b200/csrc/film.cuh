@@ -8,9 +8,9 @@
 // every pixel whose centre lies within the filter's half size, and the same weight to W
 // (HdrRgbFilm::addRgbSample, HdrRgbFilm.cpp:82-123). With the 4 x 4 filters the renderer first
 // collects every path's radiance in a per-path buffer (the shading kernel stores it when the path
-// ends, the traversal kernel adds the NEE light found at its last vertex), and one pass in path
-// order then splats all samples: consecutive paths are neighbouring pixels, so a warp's atomics
-// land in a few adjacent cache lines instead of all over the film. Samples are spread over the film's sample
+// ends, the traversal kernel adds the NEE light found at its last vertex), and one pass then gathers
+// them tile by tile (gather_samples_kernel; films more than 65,536 pixels wide or high are splatted in
+// path order instead, so that a warp's atomics land in a few adjacent cache lines). Samples are spread over the film's sample
 // window, the pixel-centre rectangle grown by the half size on every side, so that border pixels
 // see the whole filter support (TSamplingFilm::updateSampleDimensions with soft edges,
 // Engine/Source/Core/Filmic/TSamplingFilm.ipp:102-119). Here the window is cut into W x H equal

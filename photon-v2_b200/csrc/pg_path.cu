@@ -180,7 +180,8 @@ __device__ __forceinline__ void splat(const FilmView& f, uint32_t pixel, uint32_
 }
 
 // 4 x 4 filters: every path of the pass into the film, in path order (its raster position from
-// the same counter-based draws the camera ray used), radiance and weight W together.
+// the same counter-based draws the camera ray used), radiance and weight W together. Films wider or
+// higher than kGatherMaxSide; smaller ones take gather_samples_kernel.
 __global__ void __launch_bounds__(kShadeBlock)
 splat_samples_kernel(FilmView film, uint64_t seed, uint64_t first_global, uint32_t num_paths)
 {
@@ -192,6 +193,174 @@ splat_samples_kernel(FilmView film, uint64_t seed, uint64_t first_global, uint32
 		const float2 r = raster_position(film, p % wh, rng);
 		film_deposit(film, r.x, r.y, make_float4(c.x, c.y, c.z, 1.0f));
 	}
+}
+
+// The same film update, gathered: a block owns a tile of kGatherX x kGatherY pixels and, sample by
+// sample, stages the tile's cells (each pixel index owns one cell of the sample window, so a pixel
+// only sees the cells up to kGatherHalo around it) in shared memory as filter weights and FP64
+// radiance; every thread then sums its pixel's share in FP64 registers, and adds it to the film once.
+// Splatting a sample takes 64 FP64 atomics, which bound splat_samples_kernel; here a sample costs
+// its weights (1.6 times, for the tile's rim) and a look at 36 cells per pixel: a 637 x 359 render of
+// 32 samples per pixel went from 16.0 to 14.3 ms, its film from 1.9 to about 0.2 ms. Blocks in z
+// share the samples per pixel where the tiles alone would leave SMs idle.
+constexpr int kGatherX = 32, kGatherY = 16;          // tile
+constexpr int kGatherThreads = 256;                  // two pixels each: rows ty and ty + 8
+constexpr int kGatherCellsX = kGatherX + 8, kGatherCellsY = kGatherY + 8;
+constexpr int kGatherCells = kGatherCellsX * kGatherCellsY;
+constexpr int kTaps = 5;                             // pixel centres within 2 px of a point, both ends counted
+constexpr uint32_t kGatherMaxSide = 1u << 16;        // the cell range's rounding margin stays below 1/10 cell
+constexpr int kGatherSmem = kGatherCells * (2 * kTaps * 4 + 3 * 8 + 4);
+
+// The cells whose samples can reach pixels [p0, p1] of one axis: a sample at (cell + u) * s, u in
+// [0, 1), reaches the pixels p with (cell + u) * s in [p, p + 4] (the window starts 2 px before
+// the first pixel's centre). `margin` covers the rounding of the sample's raster position.
+__device__ __forceinline__ int2 cell_range(float p0, float p1, float s, uint32_t size)
+{
+	const float margin = 1e-3f + 1e-6f * p1;
+	const int lo = static_cast<int>(ceilf(p0 / s - 1.0f - margin));
+	const int hi = static_cast<int>(floorf((p1 + 4.0f) / s + margin));
+	return make_int2(max(lo, 0), min(hi, static_cast<int>(size) - 1));
+}
+
+// One axis of a sample's footprint as film_deposit computes it: the first pixel (returned) and the
+// weights of the pixels from there on, 0 past the last.
+__device__ __forceinline__ int axis_taps(const FilmView& f, float raster, uint32_t size, float* w, int stride)
+{
+	const float c = __fsub_rn(raster, 0.5f);
+	const int first = max(0, static_cast<int>(ceilf(c - f.half)));
+	const int last = min(static_cast<int>(size) - 1, static_cast<int>(floorf(c + f.half)));
+	#pragma unroll
+	for(int k = 0; k < kTaps; ++k)
+	{
+		w[k * stride] = first + k <= last ? filter_axis(f.filter, __fsub_rn(static_cast<float>(first + k), c)) : 0.0f;
+	}
+	return first;
+}
+
+__global__ void __launch_bounds__(kGatherThreads)
+gather_samples_kernel(FilmView film, uint64_t seed, uint64_t first_global, uint32_t spp)
+{
+	extern __shared__ double gather_smem[];
+	double* s_r = gather_smem;                                  // [cell] radiance
+	double* s_g = s_r + kGatherCells;
+	double* s_b = s_g + kGatherCells;
+	float* s_wx = reinterpret_cast<float*>(s_b + kGatherCells);   // [tap][cell] weights
+	float* s_wy = s_wx + kTaps * kGatherCells;
+	int* s_first = reinterpret_cast<int*>(s_wy + kTaps * kGatherCells);   // first pixel, tile-relative: x | y << 16
+
+	const int tile_x = static_cast<int>(blockIdx.x) * kGatherX, tile_y = static_cast<int>(blockIdx.y) * kGatherY;
+	const int end_x = min(tile_x + kGatherX, static_cast<int>(film.width)) - 1;
+	const int end_y = min(tile_y + kGatherY, static_cast<int>(film.height)) - 1;
+	const int2 rx = cell_range(static_cast<float>(tile_x), static_cast<float>(end_x), film.sx, film.width);
+	const int2 ry = cell_range(static_cast<float>(tile_y), static_cast<float>(end_y), film.sy, film.height);
+	const int cells_x = rx.y - rx.x + 1, cells_y = ry.y - ry.x + 1;   // at most kGatherCellsX x kGatherCellsY
+
+	// this thread's pixels and the cells that can reach them, tile-relative
+	const int px = threadIdx.x % kGatherX, py0 = threadIdx.x / kGatherX;
+	const int2 cx = cell_range(static_cast<float>(tile_x + px), static_cast<float>(tile_x + px), film.sx, film.width);
+	double sum[2][4] = {};
+
+	const uint64_t wh = static_cast<uint64_t>(film.width) * film.height;
+	for(uint32_t s = blockIdx.z; s < spp; s += gridDim.z)
+	{
+		__syncthreads();   // the previous sample's cells are read
+		for(int k = threadIdx.x; k < cells_x * cells_y; k += kGatherThreads)
+		{
+			const int x = rx.x + k % cells_x, y = ry.x + k / cells_x;
+			const int cell = (k / cells_x) * kGatherCellsX + k % cells_x;
+			const uint32_t pixel = static_cast<uint32_t>(y) * film.width + static_cast<uint32_t>(x);
+			const uint64_t p = s * wh + pixel;
+			const float4 c = film.samples[p];
+			const PathRng rng = make_rng(seed, first_global + p);
+			const float2 r = raster_position(film, pixel, rng);
+			const int fx = axis_taps(film, r.x, film.width, s_wx + cell, kGatherCells);
+			const int fy = axis_taps(film, r.y, film.height, s_wy + cell, kGatherCells);
+			s_first[cell] = static_cast<int>((static_cast<uint32_t>(fx - tile_x) & 0xFFFFu) | (static_cast<uint32_t>(fy - tile_y) << 16));
+			s_r[cell] = static_cast<double>(c.x);
+			s_g[cell] = static_cast<double>(c.y);
+			s_b[cell] = static_cast<double>(c.z);
+		}
+		__syncthreads();
+		#pragma unroll
+		for(int q = 0; q < 2; ++q)
+		{
+			const int py = py0 + q * (kGatherThreads / kGatherX);
+			if(tile_x + px > end_x || tile_y + py > end_y)
+			{
+				continue;
+			}
+			const int2 cy = cell_range(static_cast<float>(tile_y + py), static_cast<float>(tile_y + py), film.sy, film.height);
+			for(int y = cy.x; y <= cy.y; ++y)
+			{
+				for(int x = cx.x; x <= cx.y; ++x)
+				{
+					const int cell = (y - ry.x) * kGatherCellsX + (x - rx.x);
+					const int first = s_first[cell];
+					const uint32_t tx = static_cast<uint32_t>(px - static_cast<int>(static_cast<short>(first & 0xFFFF)));
+					const uint32_t ty = static_cast<uint32_t>(py - (first >> 16));
+					if(tx >= static_cast<uint32_t>(kTaps) || ty >= static_cast<uint32_t>(kTaps))
+					{
+						continue;
+					}
+					float w = __fmul_rn(s_wx[tx * kGatherCells + cell], s_wy[ty * kGatherCells + cell]);
+					if(film.filter == PG_FILTER_GAUSSIAN)
+					{
+						w = fmaxf(__fsub_rn(w, kGaussianEdge), 0.0f);
+					}
+					if(w == 0.0f)
+					{
+						continue;
+					}
+					const double dw = static_cast<double>(w);
+					sum[q][0] = fma(s_r[cell], dw, sum[q][0]);
+					sum[q][1] = fma(s_g[cell], dw, sum[q][1]);
+					sum[q][2] = fma(s_b[cell], dw, sum[q][2]);
+					sum[q][3] += dw;
+				}
+			}
+		}
+	}
+	#pragma unroll
+	for(int q = 0; q < 2; ++q)
+	{
+		const int py = py0 + q * (kGatherThreads / kGatherX);
+		if(tile_x + px > end_x || tile_y + py > end_y)
+		{
+			continue;
+		}
+		double* dst = film.sums + (static_cast<size_t>(tile_y + py) * film.width + (tile_x + px)) * kFilmChannels;
+		#pragma unroll
+		for(int k = 0; k < 4; ++k)
+		{
+			if(sum[q][k] != 0.0)
+			{
+				atomicAdd(dst + k, sum[q][k]);
+			}
+		}
+	}
+}
+
+// Gathers (or, for very wide or high films, splats) the pass's samples into the film.
+void launch_film_samples(const FilmView& film, uint64_t seed, uint64_t first_global, uint32_t spp, int grid, int sms,
+                         cudaStream_t st)
+{
+	if(film.width > kGatherMaxSide || film.height > kGatherMaxSide)
+	{
+		splat_samples_kernel<<<grid, kShadeBlock, 0, st>>>(film, seed, first_global, film.width * film.height * spp);
+		PG_CUDA_CHECK(cudaGetLastError());
+		return;
+	}
+	static const bool configured = []
+	{
+		PG_CUDA_CHECK(cudaFuncSetAttribute(gather_samples_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGatherSmem));
+		return true;
+	}();
+	(void)configured;
+	const uint32_t tx = (film.width + kGatherX - 1u) / kGatherX, ty = (film.height + kGatherY - 1u) / kGatherY;
+	// three blocks fit an SM; several rounds of them keep the last one short
+	const uint32_t split = std::min<uint32_t>(spp, std::max<uint32_t>(1u, 12u * static_cast<uint32_t>(sms) / (tx * ty)));
+	gather_samples_kernel<<<dim3(tx, ty, split), kGatherThreads, kGatherSmem, st>>>(film, seed, first_global, spp);
+	PG_CUDA_CHECK(cudaGetLastError());
 }
 
 // Previews during a render: the continuing paths of the queue the next iteration starts from,
@@ -2407,8 +2576,7 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 	{
 		if(params.filter != PG_FILTER_BOX)
 		{
-			splat_samples_kernel<<<grid, kShadeBlock, 0, st>>>(film, params.seed, first_global, static_cast<uint32_t>(total));
-			PG_CUDA_CHECK(cudaGetLastError());
+			launch_film_samples(film, params.seed, first_global, params.spp, grid, sms, st);
 		}
 	};
 
