@@ -466,7 +466,7 @@ classify_kernel(DeviceScene s_single, RenderCounters* __restrict__ c, const uint
 		uint32_t base = 0;
 		if(peers.thread_rank() == 0)
 		{
-			base = atomicAdd(&c->n_class[list], peers.size());
+			base = atomicAdd(&c->n_class[list].n, peers.size());
 		}
 		base = peers.shfl(base, 0);
 		order[list * list_capacity + base + peers.thread_rank()] = i;
@@ -488,64 +488,71 @@ __device__ __forceinline__ uint32_t alloc_slot(uint32_t* counter)
 
 // ---------------------------------------------------------------------------------------------
 
+// The start of an iteration: the queue's numbers, and camera rays of new paths into the tail of the
+// current queue (PinholeCamera::receiveRay, then BNEEPTEstimator.cpp:63-64: reversed, range
+// [0, max]). `prev` holds the previous iteration's counters and `c` this one's (two sets, by
+// parity), so that every block can derive the queue's numbers from `prev` while the first block
+// writes them to `c`.
+//
 // Training periods (guided renders that train): at position 0 the count of marked vertices starts
 // afresh; at position 1 the count of samples does, and the share of marked vertices that record a
 // sample is set so that they fill record_budget rows on average. Every marked vertex is kept with
 // the same probability, whatever the material its path reaches next (taking the first rows
 // handed out would favour the classes the shading kernel processes first).
-__global__ void prepare_kernel(RenderCounters* c, uint32_t capacity, uint32_t period_pos, uint32_t record_budget)
-{
-	if(threadIdx.x != 0 || blockIdx.x != 0)
-	{
-		return;
-	}
-	const uint32_t active = c->n_next;
-	const unsigned long long remaining = c->total_paths - c->next_path;
-	const unsigned long long room = static_cast<unsigned long long>(capacity - active);
-	const uint32_t n_new = static_cast<uint32_t>(remaining < room ? remaining : room);
-	c->n_active = active;
-	c->n_total = active + n_new;
-	c->gen_base = c->next_path;
-	c->next_path += n_new;
-	c->n_next = 0;
-	c->n_shadow_prev = c->n_shadow;
-	c->n_shadow = 0;
-	c->fetch_extend = 0;
-	c->fetch_shadow = 0;
-	c->guided_total += c->n_guided;
-	c->n_guided = 0;
-	if(period_pos == 0u)
-	{
-		c->n_marked = 0;
-	}
-	if(period_pos == 1u)
-	{
-		c->rec_keep = c->n_marked > record_budget ? static_cast<float>(record_budget) / static_cast<float>(c->n_marked)
-		                                          : 1.0f;
-		c->n_train = 0;
-	}
-	c->n_refine = 0;
-	c->n_refine_mutual = 0;
-	for(uint32_t k = 0; k < kOrderLists; ++k)
-	{
-		c->n_class[k] = 0;
-	}
-	c->rays_traced += c->n_total;
-}
-
-// Camera rays of new paths into the tail of the current queue
-// (PinholeCamera::receiveRay, then BNEEPTEstimator.cpp:63-64: reversed, range [0, max]).
+//
 // MULTI: new paths are numbered across the scenes of `batch` (scene k owns [path_first,
 // path_first + path_count)); each takes its scene's camera, film and sample numbering, and carries
 // its scene in the top bits of its meta word.
 template<bool MULTI>
 __global__ void __launch_bounds__(kShadeBlock)
-regen_kernel(const RenderCounters* __restrict__ c, Camera cam_single, FilmView film_single, uint64_t seed,
-             uint64_t first_global_single, PathBuffers cur, BatchView batch)
+begin_kernel(const RenderCounters* __restrict__ prev, RenderCounters* __restrict__ c, uint32_t capacity,
+             uint32_t period_pos, uint32_t record_budget, Camera cam_single, FilmView film_single,
+             const RenderConsts* __restrict__ k,
+             PathBuffers cur, BatchView batch)
 {
-	const uint32_t active = c->n_active;
-	const uint32_t total = c->n_total;
-	const unsigned long long base = c->gen_base;
+	const uint32_t active = prev->n_next;
+	const unsigned long long base = prev->next_path;
+	const unsigned long long remaining = prev->total_paths - base;
+	const unsigned long long room = static_cast<unsigned long long>(capacity - active);
+	const uint32_t n_new = static_cast<uint32_t>(remaining < room ? remaining : room);
+	const uint32_t total = active + n_new;
+	if(blockIdx.x == 0)
+	{
+		static_assert(kOrderLists <= kShadeBlock, "one thread per class list");
+		if(threadIdx.x < kOrderLists)
+		{
+			c->n_class[threadIdx.x].n = 0;
+		}
+		if(threadIdx.x == 0)
+		{
+			c->n_total = total;
+			c->n_next = 0;
+			c->n_shadow = 0;
+			c->n_shadow_prev = prev->n_shadow;
+			c->next_path = base + n_new;
+			c->total_paths = prev->total_paths;
+			c->rays_traced = prev->rays_traced + total;
+			c->shadow_rays = prev->shadow_rays + prev->n_shadow;   // traced in this iteration
+			c->nodes_closest = prev->nodes_closest;
+			c->tris_closest = prev->tris_closest;
+			c->nodes_any = prev->nodes_any;
+			c->tris_any = prev->tris_any;
+			c->guided_total = prev->guided_total + prev->n_guided;
+			c->iterations = prev->iterations + 1u;
+			c->pause_at = prev->pause_at;
+			c->pause_step = prev->pause_step;
+			c->error = prev->error;
+			c->fetch = 0;
+			c->n_guided = 0;
+			c->n_refine = 0;
+			c->n_refine_mutual = 0;
+			const uint32_t marked = prev->n_marked;
+			c->n_marked = period_pos == 0u ? 0u : marked;
+			c->n_train = period_pos == 1u ? 0u : prev->n_train;
+			c->rec_keep = period_pos != 1u ? prev->rec_keep
+			              : marked > record_budget ? static_cast<float>(record_budget) / static_cast<float>(marked) : 1.0f;
+		}
+	}
 	for(uint32_t i = active + blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x)
 	{
 		const unsigned long long pb = base + (i - active);
@@ -574,11 +581,11 @@ regen_kernel(const RenderCounters* __restrict__ c, Camera cam_single, FilmView f
 			p = static_cast<uint32_t>(pb);
 			cam = cam_single;
 			film = film_single;
-			first_global = first_global_single;
+			first_global = k->first_global;
 		}
 		const uint32_t wh = cam.width * cam.height;
 		const uint32_t pixel = p % wh;
-		const PathRng rng = make_rng(seed, first_global + p);
+		const PathRng rng = make_rng(k->seed, first_global + p);
 		const float2 raster = raster_position(film, pixel, rng);
 		const float rx = raster.x;
 		const float ry = raster.y;
@@ -600,6 +607,35 @@ regen_kernel(const RenderCounters* __restrict__ c, Camera cam_single, FilmView f
 		cur.ray_o[i] = make_float4(cam.pos[0], cam.pos[1], cam.pos[2], 0.0f);
 		cur.ray_d[i] = make_float4(d.x, d.y, d.z, kFloatMax);
 	}
+}
+
+// Whether every path of the render has finished.
+__host__ __device__ inline bool render_done(const RenderCounters& c)
+{
+	return c.next_path >= c.total_paths && c.n_next == 0u && c.n_shadow == 0u;
+}
+
+// The end of a period of iterations: whether the graph's loop runs another one. It ends when every
+// path has finished, on an error (an iteration with nothing in its queues before that is one), at a
+// progress point (pause_at, for renders that publish previews; the points' distance doubles up to
+// 128 iterations) and, as a backstop, after kMaxIterations.
+constexpr uint32_t kMaxIterations = 1u << 25;
+
+__global__ void end_kernel(RenderCounters* c, cudaGraphConditionalHandle loop)
+{
+	const bool pause = c->iterations >= c->pause_at;
+	if(pause)
+	{
+		c->pause_step = min(c->pause_step * 2u, 128u);
+		c->pause_at = c->iterations + c->pause_step;
+	}
+	const bool done = render_done(*c);
+	if(!done && c->n_total == 0u && c->n_shadow_prev == 0u)
+	{
+		c->error |= PG_DEV_ERR_QUEUE;
+	}
+	const bool stop = done || c->error != 0u || pause || c->iterations >= kMaxIterations;
+	cudaGraphSetConditional(loop, stop ? 0u : 1u);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -695,8 +731,7 @@ struct ShadeArgs
 	ShadowQueue   shadow;
 	RenderCounters* counters;
 	FilmView      film;
-	uint64_t      seed;
-	uint64_t      first_global;
+	const RenderConsts* consts;
 	uint32_t      max_bounces;
 	uint32_t      estimator;
 	uint32_t      width_height;
@@ -738,6 +773,12 @@ shade_kernel(ShadeArgs a)
 	// One warp sums up the list lengths (one thread loading them one after another took longer than
 	// shading a small queue).
 	__shared__ uint32_t list_end[kLists];
+	// (once per block: the loop over the items would load these from global memory for every item)
+	__shared__ RenderConsts consts;
+	if(threadIdx.x == 0)
+	{
+		consts = *a.consts;
+	}
 	if(threadIdx.x < 32u)
 	{
 		uint32_t before = 0;
@@ -745,7 +786,7 @@ shade_kernel(ShadeArgs a)
 		for(uint32_t l0 = 0; l0 < kLists; l0 += 32u)
 		{
 			const uint32_t l = l0 + threadIdx.x;
-			uint32_t end = l < kLists ? a.counters->n_class[kFirstList + l] : 0u;
+			uint32_t end = l < kLists ? a.counters->n_class[kFirstList + l].n : 0u;
 			#pragma unroll
 			for(uint32_t d = 1; d < 32u; d *= 2u)
 			{
@@ -782,7 +823,7 @@ shade_kernel(ShadeArgs a)
 		const DeviceScene& s = MULTI ? a.batch.scenes[sid].scene : a.scene;
 		const FilmView& film = MULTI ? a.batch.scenes[sid].film : a.film;
 		const uint32_t width_height = MULTI ? a.batch.scenes[sid].width_height : a.width_height;
-		const uint64_t first_global = MULTI ? a.batch.scenes[sid].first_global : a.first_global;
+		const uint64_t first_global = MULTI ? a.batch.scenes[sid].first_global : consts.first_global;
 		const float4 thr4 = ld4(a.cur.thr + i);
 		const float4 rad4 = ld4(a.cur.rad + i);
 		const float4 prev4 = ld4(a.cur.prev + i);
@@ -790,7 +831,7 @@ shade_kernel(ShadeArgs a)
 		const float4 rd = ld4(a.cur.ray_d + i);
 		const uint2 hit = a.hits[i];
 		const uint32_t pixel = p % width_height;
-		const PathRng rng = make_rng(a.seed, first_global + p);
+		const PathRng rng = make_rng(consts.seed, first_global + p);
 
 		const RGB thr_emit = RGB{thr4.x, thr4.y, thr4.z};
 		const float cont = thr4.w;
@@ -1614,7 +1655,7 @@ RenderScene::RenderScene(const SceneDesc& desc, float max_origin_abs)
 		for(int k = 0; k < 3; ++k) { m_dev.env_map.center[k] = desc.env_center[k]; }
 		m_dev.env_map.radius = static_cast<float>(std::sqrt(desc.env_area / (4.0 * 3.14159265358979323846)));
 	}
-	m_counters.resize(1);
+	m_state.resize(1);
 	PG_CUDA_CHECK(cudaStreamSynchronize(st));
 
 	m_dev.nodes = m_geometry->nodes.get();
@@ -1639,9 +1680,16 @@ RenderScene::~RenderScene()
 		cudaStreamSynchronize(m_stream);
 		cudaStreamDestroy(m_stream);
 	}
-	if(m_host_counters)
+	if(m_host_state)
 	{
-		cudaFreeHost(m_host_counters);
+		cudaFreeHost(m_host_state);
+	}
+	for(cudaEvent_t e : m_events)
+	{
+		if(e)
+		{
+			cudaEventDestroy(e);
+		}
 	}
 }
 
@@ -1651,6 +1699,7 @@ void RenderScene::ensure_capacity(uint32_t capacity, uint32_t grid)
 	{
 		return;
 	}
+	++m_buffer_generation;
 	capacity = std::max(capacity, m_capacity);
 	for(int b = 0; b < 2; ++b)
 	{
@@ -1687,6 +1736,7 @@ void RenderScene::ensure_guiding(uint32_t capacity)
 	cudaStream_t st = m_stream;
 	if(capacity > m_guide_capacity)
 	{
+		++m_buffer_generation;
 		for(int b = 0; b < 2; ++b)
 		{
 			m_gf0[b].resize(capacity);
@@ -1702,6 +1752,7 @@ void RenderScene::ensure_guiding(uint32_t capacity)
 	const uint32_t batch = std::max<uint32_t>(m_guide_params.batch, guide::kTile);
 	if(m_tdirw.size() < batch)
 	{
+		++m_buffer_generation;
 		m_tfeat.resize(static_cast<std::size_t>(batch) * 8);
 		m_traw.resize(static_cast<std::size_t>(batch) * guide::kOut);
 		m_tdirw.resize(batch);
@@ -1735,6 +1786,7 @@ void RenderScene::ensure_guiding(uint32_t capacity)
 		fill(guide::kOffW2, guide::kHidden, guide::kHidden * guide::kHidden, 1.0);
 		fill(guide::kOffW3, guide::kHidden, guide::kHidden * guide::kHidden, 1.0);
 		fill(guide::kOffW4, guide::kHidden, guide::kHidden * guide::kOut, 0.1);
+		m_buffer_generation += m_gparams.size() == 0 ? 1u : 0u;   // a reset network keeps its buffers
 		m_gparams.resize(guide::kNumParams);
 		m_gm.resize(guide::kNumParams);
 		m_gv.resize(guide::kNumParams);
@@ -1937,6 +1989,7 @@ void RenderScene::rebuild_bvh(uint32_t max_leaf_tris)
 		                              cudaMemcpyHostToDevice, st));
 		PG_CUDA_CHECK(cudaStreamSynchronize(st));
 	}
+	++m_buffer_generation;
 	m_geometry = std::move(g);
 	m_dev.nodes = m_geometry->nodes.get();
 	m_dev.tris = m_geometry->tris.get();
@@ -2248,6 +2301,8 @@ float RenderScene::render_batch(const std::vector<const RenderScene*>& scenes, c
 // split into passes of whole samples per pixel.
 constexpr unsigned long long kMaxFilteredPassPaths = 1ull << 27;
 constexpr unsigned long long kMaxBoxPassPaths = 1ull << 31;
+// Iterations up to the first progress point of a render that publishes previews.
+constexpr uint32_t kFirstPause = 16;
 
 float RenderScene::render(const RenderParams& params, double* film_sums)
 {
@@ -2287,6 +2342,60 @@ float RenderScene::render(const RenderParams& params, double* film_sums)
 	return ms;
 }
 
+namespace
+{
+
+uint64_t float_bits(float v)
+{
+	uint32_t b;
+	std::memcpy(&b, &v, sizeof(b));
+	return b;
+}
+
+}// end anonymous namespace
+
+// Captures `launches` (on the scene's stream; given the loop's handle) as the body of a loop on the
+// device and instantiates it as m_exec.
+void RenderScene::build_loop_graph(const std::function<void(cudaGraphConditionalHandle)>& launches)
+{
+	if(m_exec)
+	{
+		PG_CUDA_CHECK(cudaGraphExecDestroy(m_exec));
+		m_exec = nullptr;
+	}
+	struct GraphHolder
+	{
+		cudaGraph_t g = nullptr;
+		~GraphHolder() { if(g) { cudaGraphDestroy(g); } }
+	} holder;
+	PG_CUDA_CHECK(cudaGraphCreate(&holder.g, 0));
+	cudaGraphConditionalHandle loop;
+	PG_CUDA_CHECK(cudaGraphConditionalHandleCreate(&loop, holder.g, 1, cudaGraphCondAssignDefault));
+	cudaGraphNodeParams node{};
+	node.type = cudaGraphNodeTypeConditional;
+	node.conditional.handle = loop;
+	node.conditional.type = cudaGraphCondTypeWhile;
+	node.conditional.size = 1;
+	cudaGraphNode_t added;
+	PG_CUDA_CHECK(cudaGraphAddNode(&added, holder.g, nullptr, 0, &node));
+	PG_CUDA_CHECK(cudaStreamBeginCaptureToGraph(m_stream, node.conditional.phGraph_out[0], nullptr, nullptr, 0,
+	                                            cudaStreamCaptureModeThreadLocal));
+	try
+	{
+		launches(loop);
+	}
+	catch(...)
+	{
+		cudaGraph_t body;
+		cudaStreamEndCapture(m_stream, &body);
+		(void)cudaGetLastError();
+		throw;
+	}
+	cudaGraph_t body;
+	PG_CUDA_CHECK(cudaStreamEndCapture(m_stream, &body));
+	PG_CUDA_CHECK(cudaGraphInstantiate(&m_exec, holder.g, 0));
+}
+
 float RenderScene::render_pass(const RenderParams& params, double* film_sums, const std::vector<BatchScene>* batch)
 {
 	const bool multi = batch != nullptr;
@@ -2323,9 +2432,6 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 	const int refill = static_cast<int>(lc.refill);
 
 	cudaStream_t st = m_stream;
-	RenderCounters init{};
-	init.total_paths = total;
-	PG_CUDA_CHECK(cudaMemcpyAsync(m_counters.get(), &init, sizeof(init), cudaMemcpyHostToDevice, st));
 	PathBuffers buf[2];
 	for(int b = 0; b < 2; ++b)
 	{
@@ -2345,12 +2451,14 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 		{
 			if(m_ssid[b].size() < m_capacity)
 			{
+				++m_buffer_generation;
 				m_ssid[b].resize(m_capacity);
 			}
 			sqs[b].sid = m_ssid[b].get();
 		}
 		if(m_batch_table.size() < batch->size())
 		{
+			++m_buffer_generation;
 			m_batch_table.resize(batch->size());
 		}
 		PG_CUDA_CHECK(cudaMemcpyAsync(m_batch_table.get(), batch->data(), batch->size() * sizeof(BatchScene),
@@ -2367,6 +2475,21 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 		film.samples = m_samples.get();
 	}
 	const uint64_t first_global = params.first_sample * wh;
+	// what changes from render to render goes through device memory, so that a scene's graph serves
+	// all its renders of one shape; the counters of the iteration before the first are set 0
+	if(!m_host_state)
+	{
+		PG_CUDA_CHECK(cudaMallocHost(&m_host_state, sizeof(RenderState)));
+	}
+	RenderCounters* const host_counters = &m_host_state->counters[0];
+	*host_counters = RenderCounters{};
+	host_counters->total_paths = total;
+	host_counters->pause_at = params.progress ? kFirstPause : 0xFFFFFFFFu;
+	host_counters->pause_step = kFirstPause;
+	m_host_state->consts = RenderConsts{params.seed, first_global};
+	PG_CUDA_CHECK(cudaMemcpyAsync(m_state.get(), m_host_state, kStateHead, cudaMemcpyHostToDevice, st));
+	RenderCounters* const counters_of[2] = {&m_state.get()->counters[1], &m_state.get()->counters[0]};   // by parity
+	const RenderConsts* const consts = &m_state.get()->consts;
 	const bool counting = params.mode == PG_RENDER_COUNT;
 	// BVPTDL follows one BSDF-sampled bounce whatever the configured depth (BVPTDLEstimator.cpp:62-95)
 	const uint32_t max_bounces = params.estimator == PG_EST_BVPTDL ? 1u : params.max_bounces;
@@ -2410,7 +2533,6 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 		PG_CUDA_CHECK(cudaMemsetAsync(m_gerr.get(), 0, sizeof(uint32_t), st));
 		PG_CUDA_CHECK(cudaMemsetAsync(m_gscalars.get(), 0, 4 * sizeof(float), st));
 	}
-	RenderCounters* const d_counters = m_counters.get();
 	// the shading kernels this render's materials need
 	uint32_t kinds = m_shade_kinds;
 	if(multi)
@@ -2455,21 +2577,22 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 		const int b = q & 1;
 		const PathBuffers& cur = buf[b];
 		const PathBuffers& nxt = buf[1 - b];
+		RenderCounters* const d_counters = counters_of[b];
 		if(ev) { PG_CUDA_CHECK(cudaEventRecord(ev[0], st)); }
-		// the training samples of a period start at q = 1
-		prepare_kernel<<<1, 32, 0, st>>>(m_counters.get(), capacity, training ? static_cast<uint32_t>(q) : 2u,
-		                                 train_cap / 4u * 3u);
 		if(ev) { PG_CUDA_CHECK(cudaEventRecord(ev[1], st)); }
+		// the training samples of a period start at q = 1
+		const uint32_t pos = training ? static_cast<uint32_t>(q) : 2u;
 		if(multi)
 		{
-			regen_kernel<true><<<grid, kShadeBlock, 0, st>>>(m_counters.get(), m_dev.cam, film, params.seed, first_global,
-			                                                 cur, bview);
+			begin_kernel<true><<<grid, kShadeBlock, 0, st>>>(counters_of[1 - b], d_counters, capacity, pos,
+			                                                 train_cap / 4u * 3u, m_dev.cam, film, consts, cur, bview);
 		}
 		else
 		{
-			regen_kernel<false><<<grid, kShadeBlock, 0, st>>>(m_counters.get(), m_dev.cam, film, params.seed, first_global,
-			                                                  cur, bview);
+			begin_kernel<false><<<grid, kShadeBlock, 0, st>>>(counters_of[1 - b], d_counters, capacity, pos,
+			                                                  train_cap / 4u * 3u, m_dev.cam, film, consts, cur, bview);
 		}
+		PG_CUDA_CHECK(cudaGetLastError());
 		if(ev) { PG_CUDA_CHECK(cudaEventRecord(ev[2], st)); }
 		const ShadowQueue& sq = sqs[b];   // this iteration's NEE segments
 		// closest hits of this iteration and the previous iteration's NEE segments (whose
@@ -2498,8 +2621,8 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 			                      &d_counters->n_guided, m_graw.get());
 		}
 		if(ev) { PG_CUDA_CHECK(cudaEventRecord(ev[4], st)); }
-		ShadeArgs sa{m_dev, cur, nxt, m_hits.get(), sq, m_counters.get(), film, params.seed, first_global,
-		             max_bounces, params.estimator, static_cast<uint32_t>(wh)};
+		ShadeArgs sa{m_dev, cur, nxt, m_hits.get(), sq, d_counters, film, consts, max_bounces, params.estimator,
+		             static_cast<uint32_t>(wh)};
 		sa.guide = gargs_b;
 		sa.refine.mode = params.refine_mode;
 		sa.refine.delta = params.refine_delta;
@@ -2580,13 +2703,7 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 		}
 	};
 
-	if(!m_host_counters)
-	{
-		PG_CUDA_CHECK(cudaMallocHost(&m_host_counters, sizeof(RenderCounters)));
-	}
-	RenderCounters* const host_counters = m_host_counters;
-
-	// a preview of the film at a batch boundary (the stream is idle there); see RenderProgress
+	// a preview of the film at a progress point (the stream is idle there); see RenderProgress
 	if(params.progress && m_inflight.size() < wh)
 	{
 		m_inflight.resize(wh);
@@ -2601,7 +2718,7 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 			if(box)
 			{
 				PG_CUDA_CHECK(cudaMemsetAsync(m_inflight.get(), 0, wh * sizeof(uint32_t), st));
-				count_inflight_kernel<<<grid, kShadeBlock, 0, st>>>(buf[0].path, m_counters.get(), pixels, m_inflight.get());
+				count_inflight_kernel<<<grid, kShadeBlock, 0, st>>>(buf[0].path, counters_of[1], pixels, m_inflight.get());
 				PG_CUDA_CHECK(cudaGetLastError());
 			}
 			develop_preview_kernel<<<grid, kShadeBlock, 0, st>>>(film_sums, m_inflight.get(), pixels, params.spp,
@@ -2614,73 +2731,72 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 			pr.published(hc.next_path - hc.n_next, total);
 		}
 	};
-	cudaEvent_t e0, e1;
-	PG_CUDA_CHECK(cudaEventCreate(&e0));
-	PG_CUDA_CHECK(cudaEventCreate(&e1));
+	for(cudaEvent_t& e : m_events)
+	{
+		if(!e)
+		{
+			PG_CUDA_CHECK(cudaEventCreate(&e));
+		}
+	}
+	const cudaEvent_t e0 = m_events[0], e1 = m_events[1];
 	unsigned long long iterations = 0;
-	const unsigned long long max_iterations = 1ull << 25;
 	bool done = false;
 	for(double& k : m_kernel_ms) { k = 0.0; }
 
 	if(params.mode == PG_RENDER_GRAPH)
 	{
-		// One graph = one period: two iterations (ping -> pong -> ping), four when training. The
-		// launch sequence only depends on whether guiding and training run, so the executable
-		// graph of the previous render is updated with this render's kernel arguments and
-		// instantiated again only when its topology changed.
-		cudaGraph_t graph;
-		PG_CUDA_CHECK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-		for(int q = 0; q < period; ++q)
+		// One graph = a loop on the device over periods (two iterations, ping -> pong -> ping; four when
+		// training): the last kernel of a period decides whether another follows, so that no
+		// iteration runs after the last path and the host only waits. (Periods launched by the host
+		// in batches of 4, 8, ... ran up to 14 empty iterations on short renders: a 64 x 48 thumbnail
+		// took 24 iterations for its 9.) The graph is built again only when something its launches
+		// were given has changed.
+		std::vector<uint64_t> key = {static_cast<uint64_t>(period), guided, training, multi, kinds, static_cast<uint64_t>(grid),
+		                             capacity, static_cast<uint64_t>(refill), m_order_list, max_bounces, params.estimator, wh,
+		                             params.refine_mode, float_bits(params.refine_delta), params.refine_iters,
+		                             m_dev.env_map.exact, guide_depth, train_cap, bview.count, m_buffer_generation, params.filter,
+		                             reinterpret_cast<uint64_t>(film.sums), reinterpret_cast<uint64_t>(film.samples)};
+		if(guided)
 		{
-			iteration(q, nullptr);
-		}
-		PG_CUDA_CHECK(cudaStreamEndCapture(st, &graph));
-		const int key = (guided ? 1 : 0) | (training ? 2 : 0) | (multi ? 4 : 0) | static_cast<int>(kinds << 3);
-		bool updated = false;
-		if(m_exec && m_exec_key == key)
-		{
-			cudaGraphExecUpdateResultInfo info;
-			updated = cudaGraphExecUpdate(m_exec, graph, &info) == cudaSuccess;
-			if(!updated)
+			for(float v : {m_guide_params.alpha, m_guide_params.lr, m_guide_params.clamp})
 			{
-				(void)cudaGetLastError();   // a failed update is not sticky; instantiate anew
+				key.push_back(float_bits(v));
 			}
 		}
-		if(!updated)
+		if(!m_exec || m_exec_key != key)
 		{
-			if(m_exec)
+			build_loop_graph([&](cudaGraphConditionalHandle loop)
 			{
-				PG_CUDA_CHECK(cudaGraphExecDestroy(m_exec));
-				m_exec = nullptr;
-			}
-			PG_CUDA_CHECK(cudaGraphInstantiate(&m_exec, graph, 0));
+				for(int q = 0; q < period; ++q)
+				{
+					iteration(q, nullptr);
+				}
+				end_kernel<<<1, 1, 0, st>>>(counters_of[1], loop);
+				PG_CUDA_CHECK(cudaGetLastError());
+			});
 			m_exec_key = key;
 		}
-		PG_CUDA_CHECK(cudaGraphDestroy(graph));
-		cudaGraphExec_t exec = m_exec;
 		PG_CUDA_CHECK(cudaEventRecord(e0, st));
 		add_box_weights();
-		int batch = 4;
-		while(!done && iterations < max_iterations)
+		while(!done)
 		{
-			for(int k = 0; k < batch; ++k)
-			{
-				PG_CUDA_CHECK(cudaGraphLaunch(exec, st));
-			}
-			iterations += static_cast<unsigned long long>(period) * batch;
-			PG_CUDA_CHECK(cudaMemcpyAsync(host_counters, m_counters.get(), sizeof(RenderCounters), cudaMemcpyDeviceToHost, st));
+			PG_CUDA_CHECK(cudaGraphLaunch(m_exec, st));
+			PG_CUDA_CHECK(cudaMemcpyAsync(host_counters, counters_of[1], kCountersHead, cudaMemcpyDeviceToHost, st));
 			PG_CUDA_CHECK(cudaStreamSynchronize(st));
-			done = host_counters->next_path >= host_counters->total_paths && host_counters->n_next == 0 &&
-			       host_counters->n_shadow == 0;
-			if(host_counters->error)
+			iterations = host_counters->iterations;
+			done = render_done(*host_counters);
+			if(host_counters->error || iterations >= kMaxIterations)
 			{
 				break;
 			}
-			if(params.progress && !done)
+			if(!done)
 			{
+				if(!params.progress)
+				{
+					break;   // only progress points end the loop before the last path
+				}
 				publish_preview(*host_counters);
 			}
-			batch = std::min(batch * 2, 64);
 		}
 		splat_samples();
 		PG_CUDA_CHECK(cudaEventRecord(e1, st));
@@ -2695,11 +2811,12 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 		for(cudaEvent_t& e : ev) { PG_CUDA_CHECK(cudaEventCreate(&e)); }
 		PG_CUDA_CHECK(cudaEventRecord(e0, st));
 		add_box_weights();
-		while(!done && iterations < max_iterations)
+		while(!done && iterations < kMaxIterations)
 		{
-			iteration(static_cast<int>(iterations % static_cast<unsigned long long>(period)), timing ? ev : nullptr);
+			const int q = static_cast<int>(iterations % static_cast<unsigned long long>(period));
+			iteration(q, timing ? ev : nullptr);
 			++iterations;
-			PG_CUDA_CHECK(cudaMemcpyAsync(host_counters, m_counters.get(), sizeof(RenderCounters), cudaMemcpyDeviceToHost, st));
+			PG_CUDA_CHECK(cudaMemcpyAsync(host_counters, counters_of[q & 1], kCountersHead, cudaMemcpyDeviceToHost, st));
 			PG_CUDA_CHECK(cudaStreamSynchronize(st));
 			if(timing)
 			{
@@ -2712,8 +2829,7 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 					m_kernel_ms[slot[k]] += ms;
 				}
 			}
-			done = host_counters->next_path >= host_counters->total_paths && host_counters->n_next == 0 &&
-			       host_counters->n_shadow == 0;
+			done = render_done(*host_counters);
 			if(host_counters->error)
 			{
 				break;
@@ -2727,23 +2843,23 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 
 	float ms = 0.0f;
 	PG_CUDA_CHECK(cudaEventElapsedTime(&ms, e0, e1));
-	cudaEventDestroy(e0);
-	cudaEventDestroy(e1);
 	const RenderCounters final_counters = *host_counters;
 
 	m_last_rays = final_counters.rays_traced;
 	m_last_shadow = final_counters.shadow_rays;
 	m_last_iterations = iterations;
 	{
-		// prepare, regen, trace + classify, shade per material kind (+ refine in the iterative
+		// begin, trace + classify, shade per material kind (+ refine in the iterative
 		// mode); guide query + forward; training: weight sums (and clamp), forward, backward, Adam,
 		// step, repack, loss
-		const unsigned long long per_iteration = 5ull + ((kinds >> kShadeConductor) & 1u) + ((kinds >> kShadeDielectric) & 1u) +
+		const unsigned long long per_iteration = 4ull + ((kinds >> kShadeConductor) & 1u) + ((kinds >> kShadeDielectric) & 1u) +
 		                                         (params.refine_mode == PG_REFINE_ITERATIVE ? 1ull : 0ull) +
 		                                         (guided ? 2ull : 0ull);
 		const unsigned long long per_step = training ? (m_guide_params.clamp > 0.0f ? 8ull : 6ull) : 0ull;
-		// + one training step per training period, + the film's box-weight or splat launch
-		m_last_launches = iterations * per_iteration + iterations / kTrainPeriod * per_step + 1ull;
+		// + the end of every period (graph mode), one training step per training period, and the film's
+		// box-weight or splat launch
+		const unsigned long long ends = params.mode == PG_RENDER_GRAPH ? iterations / static_cast<unsigned long long>(period) : 0ull;
+		m_last_launches = iterations * per_iteration + ends + iterations / kTrainPeriod * per_step + 1ull;
 	}
 	m_last_counts[0] = final_counters.nodes_closest;
 	m_last_counts[1] = final_counters.tris_closest;

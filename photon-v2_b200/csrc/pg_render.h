@@ -2,15 +2,17 @@
 //
 // One render = W x H x spp independent paths of the BNEEPT (or BVPT) estimator. Paths live in a
 // fixed-capacity pool of slots; every iteration
-//   prepare  -> compacts bookkeeping and decides how many new camera paths join,
-//   regen    -> writes the new camera rays into the free tail of the ray queue,
-//   extend   -> closest hit for every queued ray (pg_trace.cu),
+//   begin    -> decides how many new camera paths join and writes their rays into the free tail of
+//               the ray queue,
+//   trace    -> closest hit for every queued ray, and any hit for the shadow rays of the previous
+//               iteration (pg_trace.cu); unoccluded contributions are added to their path (or
+//               straight to the film for paths that ended at that vertex),
+//   classify -> lists the queue's slots per shading class,
 //   shade    -> emission / NEE / BSDF sampling / Russian roulette per hit, writing continuing
 //               paths compacted (warp-aggregated) into the other buffer and shadow rays into the
 //               shadow queue,
-//   shadow   -> any hit for the shadow queue; unoccluded contributions are added to the path
-//               (or straight to the film for paths that ended at that vertex),
-// and the buffers swap. Two iterations (ping and pong) are captured in one CUDA graph.
+//   refine   -> moves the new rays' origins off their surfaces,
+// and the buffers swap. Two iterations (ping and pong) are the body of a loop in one CUDA graph.
 #pragma once
 
 #include "bsdf.cuh"
@@ -19,6 +21,7 @@
 #include "pg_common.cuh"
 #include "pg_geometry.h"
 
+#include <cstddef>
 #include <cstdint>
 #include <functional>
 #include <memory>
@@ -200,34 +203,57 @@ constexpr uint32_t kShadeClasses = 6;
 constexpr uint32_t kClassLists = 16;
 constexpr uint32_t kOrderLists = kShadeClasses * kClassLists;
 
-// Counters shared by the kernels of one render (device memory).
-struct alignas(16) RenderCounters
+// Counters shared by the kernels of one iteration (device memory). Two sets alternate: an iteration
+// derives its own from the previous one's (begin_kernel), so the counts that run over the whole
+// render are carried along.
+// The counters that every warp of a kernel adds to lie on cache lines of their own: atomics on one
+// line queue up behind each other (with all but the class lists on one line, shading and refinery of the
+// bench scene took 14 % longer).
+struct alignas(128) RenderCounters
 {
-	uint32_t n_active;      // continuing paths at the head of the current queue
-	uint32_t n_total;       // n_active + newly generated paths this iteration
-	uint32_t n_next;        // compaction counter of the next queue
-	uint32_t n_shadow;      // shadow queue length (records made this iteration)
+	uint32_t n_total;       // paths in the queue: the previous iteration's n_next and new ones
+	uint32_t n_shadow_prev; // records made by the previous iteration, traced by this one's trace_kernel
 	unsigned long long next_path;   // next path index to generate
 	unsigned long long total_paths;
-	unsigned long long gen_base;    // first path index generated this iteration
 	unsigned long long rays_traced; // closest-hit rays (extension + camera)
 	unsigned long long shadow_rays;
 	unsigned long long nodes_closest, tris_closest;   // counting mode only
 	unsigned long long nodes_any, tris_any;
-	unsigned long long guided_total;   // guided vertices over the whole render
+	unsigned long long guided_total;   // guided vertices of earlier iterations
+	uint32_t iterations;     // begun so far
+	uint32_t pause_at;       // progress point: the device loop ends at this many iterations
+	uint32_t pause_step;     // distance from the last progress point to pause_at
 	uint32_t error;
-	uint32_t pad;
-	uint32_t fetch_extend;   // dynamic-fetch cursors of the persistent traversal kernels,
-	uint32_t fetch_shadow;   // zeroed by prepare_kernel at the start of every iteration
-	uint32_t n_guided;       // guided vertices this iteration (network rows)
-	uint32_t n_train;        // training samples recorded this iteration (may exceed the batch)
-	uint32_t n_shadow_prev;  // records made by the previous iteration, traced by this one's trace_kernel
-	uint32_t n_class[kOrderLists];   // closest-hit results per shading-class list (classify_kernel)
-	uint32_t n_refine;       // surface-refinery requests this iteration: one-sided escapes
-	uint32_t n_refine_mutual;// and escapes towards a light-triangle point
-	uint32_t n_marked;       // guided vertices marked for training samples in this training period
 	float    rec_keep;       // probability that a marked vertex's sample is recorded (fits the batch)
+	alignas(128) uint32_t n_next;       // compaction counter of the next queue
+	alignas(128) uint32_t n_shadow;     // shadow queue length (records made this iteration)
+	alignas(128) uint32_t n_refine;     // surface-refinery requests this iteration: one-sided escapes
+	alignas(128) uint32_t n_refine_mutual;// and escapes towards a light-triangle point
+	alignas(128) uint32_t fetch;        // dynamic-fetch cursor of trace_kernel
+	alignas(128) uint32_t n_guided;     // guided vertices this iteration (network rows)
+	alignas(128) uint32_t n_train;      // training samples recorded this period (may exceed the batch)
+	alignas(128) uint32_t n_marked;     // guided vertices marked for training samples in this training period
+	// closest-hit results per shading-class list (classify_kernel)
+	struct alignas(128) ListLength { uint32_t n; } n_class[kOrderLists];
 };
+
+// What differs between renders of one scene and shape, read by the kernels from device memory so
+// that their launches (and the graph that holds them) stay the same.
+struct RenderConsts
+{
+	uint64_t seed;
+	uint64_t first_global;   // global index of path 0
+};
+
+struct RenderState
+{
+	RenderConsts   consts;
+	RenderCounters counters[2];
+};
+// What a render uploads at its start (the constants, and set 0 as the counters of the iteration before
+// its first) and reads back of a counter set: all but the class lists.
+constexpr std::size_t kCountersHead = offsetof(RenderCounters, n_class);
+constexpr std::size_t kStateHead = offsetof(RenderState, counters) + kCountersHead;
 
 // Surface-refinery requests of one iteration (iterative refine mode). The shading kernel leaves
 // the hit point and triangle in the ray slot it fills and queues the slot; the refinery kernel
@@ -407,6 +433,7 @@ public:
 private:
 	float render_pass(const RenderParams& params, double* film_device, const std::vector<BatchScene>* batch = nullptr);
 	void ensure_capacity(uint32_t capacity, uint32_t grid);
+	void build_loop_graph(const std::function<void(cudaGraphConditionalHandle)>& launches);
 	// Coordinate descent over the launch shapes (pool depth, refill threshold, blocks per SM, and
 	// optionally leaf size), `measure` giving a candidate's calibration milliseconds; the winner is
 	// set on this scene.
@@ -443,7 +470,7 @@ private:
 	DeviceBuffer<uint32_t> m_ssid[2];    // multi-scene renders: scene of each NEE record
 	DeviceBuffer<BatchScene> m_batch_table;
 	uint32_t m_order_list = 0;
-	DeviceBuffer<RenderCounters> m_counters;
+	DeviceBuffer<RenderState> m_state;
 
 	// learned guiding
 	GuideParams m_guide_params;
@@ -465,11 +492,13 @@ private:
 
 	// the scene's own stream: renders of different scenes, from different host threads, overlap
 	cudaStream_t m_stream = nullptr;
-	// pinned readback of the counters, and the instantiated two-iteration graph of the last
-	// render (kept across renders and updated in place when only kernel arguments change)
-	RenderCounters* m_host_counters = nullptr;
+	// pinned staging of m_state, the render's two timing events, and the instantiated loop graph of the
+	// last render with everything its launches were given (kept across renders)
+	RenderState* m_host_state = nullptr;
+	cudaEvent_t m_events[2] = {nullptr, nullptr};
 	cudaGraphExec_t m_exec = nullptr;
-	int m_exec_key = -1;
+	std::vector<uint64_t> m_exec_key;
+	uint64_t m_buffer_generation = 0;   // counts reallocations of buffers that a graph's launches name
 
 	unsigned long long m_last_rays = 0, m_last_shadow = 0, m_last_iterations = 0, m_last_launches = 0;
 	unsigned long long m_last_counts[4] = {0, 0, 0, 0};

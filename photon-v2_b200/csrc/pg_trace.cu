@@ -272,12 +272,15 @@ trace_kernel(const WideNode* __restrict__ nodes, const LeafTri* __restrict__ tri
              const uint32_t* __restrict__ meta, const uint32_t* __restrict__ shadow_sid, BatchView batch,
              const float4* __restrict__ st, float4* __restrict__ train_dirw)
 {
-	const uint32_t n_closest = counters->n_total;
-	const uint32_t n_shadow = counters->n_shadow_prev;
-	if(blockIdx.x == 0 && threadIdx.x == 0)
+	// the queue lengths, in shared memory: they are looked at when a ray is fetched or handed over, and the
+	// loop in between has no register to spare
+	__shared__ uint32_t n_closest, n_rays;
+	if(threadIdx.x == 0)
 	{
-		counters->shadow_rays += n_shadow;
+		n_closest = counters->n_total;
+		n_rays = counters->n_total + counters->n_shadow_prev;
 	}
+	__syncthreads();
 	auto scene_of = [&](uint32_t i) -> uint32_t
 	{
 		return i < n_closest ? __ldg(meta + i) >> kMetaSceneShift : __ldg(shadow_sid + (i - n_closest));
@@ -316,7 +319,7 @@ trace_kernel(const WideNode* __restrict__ nodes, const LeafTri* __restrict__ tri
 	uint32_t err = 0, node_count[2] = {0u, 0u}, tri_count[2] = {0u, 0u};
 	if constexpr(MULTI)
 	{
-		traverse_persistent<false, COUNT, true, true>(nodes, tris, n_closest + n_shadow, &counters->fetch_extend,
+		traverse_persistent<false, COUNT, true, true>(nodes, tris, n_rays, &counters->fetch,
 			[&](uint32_t i, float4* a, float4* b, const WideNode** ln, const LeafTri** lt)
 			{
 				fetch_ray(i, a, b);
@@ -328,7 +331,7 @@ trace_kernel(const WideNode* __restrict__ nodes, const LeafTri* __restrict__ tri
 	}
 	else
 	{
-		traverse_persistent<false, COUNT, true>(nodes, tris, n_closest + n_shadow, &counters->fetch_extend,
+		traverse_persistent<false, COUNT, true>(nodes, tris, n_rays, &counters->fetch,
 			fetch_ray, finish, &err, node_count, tri_count, n_closest, min_idle);
 	}
 	if(COUNT)

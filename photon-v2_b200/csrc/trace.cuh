@@ -433,10 +433,10 @@ template<bool ANY_HIT, bool COUNT, bool MIXED = false, bool MULTI = false, class
 __device__ __forceinline__ void traverse_persistent(
 	const WideNode* __restrict__ scene_nodes,
 	const LeafTri* __restrict__ scene_tris,
-	uint32_t n, uint32_t* __restrict__ next_ray,
+	const uint32_t& n, uint32_t* __restrict__ next_ray,
 	Fetch fetch, Finish finish,
 	uint32_t* out_error, uint32_t* node_count = nullptr, uint32_t* tri_count = nullptr,
-	uint32_t n_closest = 0, int min_idle = kRefillMinIdle)
+	const uint32_t& n_closest = 0u, int min_idle = kRefillMinIdle)
 {
 	// [entry][thread]: a lane's entries are 1 KB apart, so lanes at any depths hit distinct banks
 	__shared__ uint2 s_stack[kSharedStack][kTraversalBlock];
