@@ -227,7 +227,7 @@ struct alignas(128) RenderCounters
 	float    rec_keep;       // probability that a marked vertex's sample is recorded (fits the batch)
 	alignas(128) uint32_t n_next;       // compaction counter of the next queue
 	alignas(128) uint32_t n_shadow;     // shadow queue length (records made this iteration)
-	alignas(128) uint32_t n_refine;     // surface-refinery requests this iteration: one-sided escapes
+	alignas(128) uint32_t n_refine;     // queued refinery requests of NEE segments: one-sided escapes
 	alignas(128) uint32_t n_refine_mutual;// and escapes towards a light-triangle point
 	alignas(128) uint32_t fetch;        // dynamic-fetch cursor of trace_kernel
 	alignas(128) uint32_t n_guided;     // guided vertices this iteration (network rows)
@@ -255,15 +255,16 @@ struct RenderState
 constexpr std::size_t kCountersHead = offsetof(RenderCounters, n_class);
 constexpr std::size_t kStateHead = offsetof(RenderState, counters) + kCountersHead;
 
-// Surface-refinery requests of one iteration (iterative refine mode). The shading kernel leaves
-// the hit point and triangle in the ray slot it fills and queues the slot; the refinery kernel
-// replaces them with the refined origin and range. `single` entries are (slot | kind << 31):
-// kind 0 = a continuation ray in the next path buffer, 1 = a shadow ray towards a direction
-// (environment light); `mutual` entries are shadow rays towards a point on a light triangle.
+// Surface-refinery requests of one iteration (iterative refine mode). The shading kernel leaves the hit
+// point and triangle in the ray slot it fills; the refinery kernel replaces them with the refined
+// origin and range. Every slot of the next path buffer is one such request. NEE segments are queued in
+// scenes with an environment, whose shadow records towards a direction (`single`) and towards a point
+// on a light triangle (`mutual`) are refined by different loops; without one every record of the
+// shadow queue is of the second kind and both lists are null.
 struct RefineQueue
 {
-	uint32_t* single;
-	uint32_t* mutual;
+	uint32_t* single = nullptr;
+	uint32_t* mutual = nullptr;
 };
 
 // Per-path state, one buffer of the ping-pong pair (structure of arrays).

@@ -50,8 +50,7 @@ __device__ __forceinline__ RefineRay make_refine_ray(const TriVerts& tri, V3 d)
 	return q;
 }
 
-// Same bits as the full watertight test of a ray from o along the RefineRay's direction. Inlined
-// into the out-of-line offset functions below, which keep the shade kernel's own code small.
+// Same bits as the full watertight test of a ray from o along the RefineRay's direction.
 __device__ __forceinline__ bool reintersect(const RefineRay& q, V3 o, float min_t, float max_t, float* out_t)
 {
 	float b0, b1, b2;
@@ -70,7 +69,7 @@ struct OffsetResult
 // iterativeOffset (SurfaceHitRefinery.cpp:62-153). Triangles always pass canVerifyOffset
 // (planar, triangular face topology), so the empirical fallback never applies. `iters` is the
 // number of bisection refinements (EngineInitSettings::numIterativeSurfaceRefinements).
-static __device__ __noinline__ OffsetResult iterative_offset(V3 pos, V3 ng, const TriVerts& tri, V3 dir, int iters = 1)
+__device__ __forceinline__ OffsetResult iterative_offset(V3 pos, V3 ng, const TriVerts& tri, V3 dir, int iters = 1)
 {
 	const V3 offset_dir = dot(ng, dir) > 0.0f ? ng : -ng;
 	const V3 escape_dir = normalize(dir);
@@ -121,7 +120,7 @@ static __device__ __noinline__ OffsetResult iterative_offset(V3 pos, V3 ng, cons
 
 // iterativeMutualOffset (SurfaceHitRefinery.cpp:155-263): escape X towards X2, then shorten the
 // segment until it no longer touches X2's triangle.
-static __device__ __noinline__ OffsetResult iterative_mutual_offset(
+__device__ __forceinline__ OffsetResult iterative_mutual_offset(
 	V3 pos, V3 ng, const TriVerts& tri,
 	V3 pos2, const TriVerts& tri2, int iters = 1)
 {
