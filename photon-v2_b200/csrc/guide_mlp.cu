@@ -1,9 +1,13 @@
 // Guiding network on the 5th-generation tensor cores: fused forward pass of the whole MLP with
 // tcgen05.mma (BF16 operands in shared memory, FP32 accumulators in tensor memory).
 //
-// Two CTAs of 256 threads per SM walk 128-row tiles of queries; each row is owned by two threads
-// (part 0: threads 0-127, part 1: threads 128-255, thread t and t + 128 on row t), so that the
-// per-row work between the MMAs is split in two and each SM has 16 warps to hide its latency.
+// One CTA per SM, of kTeams teams of 256 threads that share the weights in shared memory; each team
+// walks 128-row tiles of queries on its own (its barriers are named, its accumulator and mbarrier its
+// own). A tile is a chain of dependent MMA groups and per-row work, so the tiles in flight on an SM are
+// what hides its latency: three teams instead of two one-team CTAs took a 192-sample guided Cornell
+// render from 19.85 to 19.0 ms; two teams were as slow as the two CTAs, a fourth gave no more. Each row
+// is owned by two threads (part 0: threads 0-127, part 1: threads 128-255, thread t and t + 128 on row
+// t), so that the per-row work between the MMAs is split in two.
 // Per tile:
 //   1. the two threads of a row one-blob encode its inputs (alternating inputs) into the A
 //      operand buffer (BF16, 224 columns, fed to the MMAs in two K halves);
@@ -43,9 +47,12 @@ namespace
 
 using namespace tc;
 
-constexpr int kThreads = 256;                 // two threads per tile row
-constexpr int kParts = kThreads / kTile;
-constexpr uint32_t kTmemCols = 128;   // power of two >= 64 accumulator columns
+constexpr int kTeamThreads = 256;             // two threads per tile row
+constexpr int kParts = kTeamThreads / kTile;
+constexpr int kTeams = 3;
+constexpr int kThreads = kTeams * kTeamThreads;
+constexpr uint32_t kTmemCols = 256;   // power of two >= 64 accumulator columns per team
+static_assert(kTeams * kHidden <= static_cast<int>(kTmemCols), "tensor memory");
 static_assert(kParts == 2 && kHidden == 64 && kLobes == 8 && kOut == 40 && kOutPad == 48,
               "the column split below assumes two parts, 64 hidden units and 8 lobes");
 
@@ -62,22 +69,39 @@ constexpr int kOffImgBias = kOffImgW4 + kW4Bytes;   // FP32 biases: 4 x 64 + 48
 constexpr int kBiasCount = kHiddenLayers * kHidden + kOutPad;
 constexpr int kImageBytes = kOffImgBias + kBiasCount * 4;   // 60,576
 
-// ---- activation buffers
-// The input layer is fed in two K halves (one-blob inputs 0-3, then 4-6) so that the A buffer is
-// 32 KB and two CTAs fit on an SM.
+// ---- activation buffer of each team
+// The input layer is fed in two K halves (one-blob inputs 0-3, then 4-6), so that a tile takes 32 KB;
+// the hidden layers overwrite it in place, each after the MMAs that read it have completed.
 constexpr int kInHalf0 = 4 * kBins;                 // 128 columns
 constexpr int kInHalf1 = kIn - kInHalf0;            //  96 columns
-constexpr int kActInBytes = kTile * kInHalf0 * 2;   // 32,768: input half, later hidden ping
-constexpr int kActHBytes = kTile * kHidden * 2;     // 16,384: hidden pong
+constexpr int kActBytes = kTile * kInHalf0 * 2;     // 32,768
 constexpr int kOffSmemImage = 0;
-constexpr int kOffSmemActIn = (kImageBytes + 1023) / 1024 * 1024;
-constexpr int kOffSmemActH = kOffSmemActIn + kActInBytes;
-constexpr int kOffSmemXch = kOffSmemActH + kActHBytes;         // [part][row] float2: softmax max, sum
-constexpr int kOffSmemBar = kOffSmemXch + kParts * kTile * 8;  // 8-byte aligned
-constexpr int kOffSmemTmem = kOffSmemBar + 8;
+constexpr int kOffSmemAct = (kImageBytes + 1023) / 1024 * 1024;
+constexpr int kOffSmemXch = kOffSmemAct + kTeams * kActBytes;           // [team][part][row] float2: softmax max, sum
+constexpr int kOffSmemBar = kOffSmemXch + kTeams * kParts * kTile * 8;  // one mbarrier per team
+constexpr int kOffSmemTmem = kOffSmemBar + kTeams * 8;
 constexpr int kSmemBytes = kOffSmemTmem + 8;
-static_assert(kImageBytes % 16 == 0 && kOffSmemActH % 16 == 0 && kOffSmemBar % 8 == 0, "alignment");
+static_assert(kImageBytes % 16 == 0 && kActBytes % 1024 == 0 && kOffSmemBar % 8 == 0, "alignment");
 static_assert(kSmemBytes <= 227 * 1024, "shared memory");
+
+// A barrier among one team's threads.
+__device__ __forceinline__ void team_sync(uint32_t team)
+{
+	asm volatile("barrier.cta.sync %0, %1;" :: "r"(team + 1u), "r"(static_cast<uint32_t>(kTeamThreads)) : "memory");
+}
+
+// The same, returning whether `p` held for any of them.
+__device__ __forceinline__ bool team_sync_or(uint32_t team, bool p)
+{
+	uint32_t any;
+	asm volatile("{\n\t"
+	             ".reg .pred a, b;\n\t"
+	             "setp.ne.u32 a, %3, 0;\n\t"
+	             "barrier.cta.red.or.pred b, %1, %2, a;\n\t"
+	             "selp.u32 %0, 1, 0, b;\n\t"
+	             "}" : "=r"(any) : "r"(team + 1u), "r"(static_cast<uint32_t>(kTeamThreads)), "r"(p ? 1u : 0u) : "memory");
+	return any != 0u;
+}
 
 // Writes 8 consecutive K values of row r (k0 multiple of 8) of an A-layout buffer.
 __device__ __forceinline__ void store_row8(unsigned char* buf, uint32_t r, uint32_t k0, const float* v)
@@ -92,15 +116,16 @@ __device__ __forceinline__ void store_row8(unsigned char* buf, uint32_t r, uint3
 
 // ---- the fused forward kernel
 
-__global__ void __launch_bounds__(kThreads, 2)
+__global__ void __launch_bounds__(kThreads, 1)
 mlp_forward_kernel(const unsigned char* __restrict__ image, const float* __restrict__ features,
                    uint32_t n_max, const uint32_t* __restrict__ d_n, float* __restrict__ out_raw,
                    float* __restrict__ out_mix, __nv_bfloat16* __restrict__ out_acts, uint32_t* __restrict__ error)
 {
 	const uint32_t n = d_n ? min(*d_n, n_max) : n_max;
 	extern __shared__ __align__(128) unsigned char smem[];
-	const uint32_t tid = threadIdx.x;
-	const uint32_t warp = tid >> 5;
+	const uint32_t team = threadIdx.x / kTeamThreads;
+	const uint32_t tid = threadIdx.x % kTeamThreads;
+	const uint32_t warp = threadIdx.x >> 5;
 	const uint32_t r = tid & (kTile - 1);   // the tile row this thread works on
 	const uint32_t part = tid / kTile;      // which half of the row's columns / lobes
 
@@ -108,12 +133,12 @@ mlp_forward_kernel(const unsigned char* __restrict__ image, const float* __restr
 	{
 		const uint4* src = reinterpret_cast<const uint4*>(image);
 		uint4* dst = reinterpret_cast<uint4*>(smem + kOffSmemImage);
-		for(uint32_t i = tid; i < kImageBytes / 16; i += kThreads)
+		for(uint32_t i = threadIdx.x; i < kImageBytes / 16; i += kThreads)
 		{
 			dst[i] = __ldg(src + i);
 		}
 	}
-	const uint32_t bar = smem_u32(smem + kOffSmemBar);
+	const uint32_t bar = smem_u32(smem + kOffSmemBar + team * 8u);
 	uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kOffSmemTmem);
 	if(tid == 0)
 	{
@@ -129,20 +154,21 @@ mlp_forward_kernel(const unsigned char* __restrict__ image, const float* __restr
 	fence_before_sync();
 	__syncthreads();
 	fence_after_sync();
-	const uint32_t tmem = *tmem_slot;
+	const uint32_t tmem_base = *tmem_slot;
+	const uint32_t tmem = tmem_base + team * static_cast<uint32_t>(kHidden);   // this team's columns
 	const uint32_t tmem_row = tmem + (((warp & 3u) * 32u) << 16);   // this warp's 32 lanes, column 0
 
 	const float* bias = reinterpret_cast<const float*>(smem + kOffImgBias);
-	unsigned char* act_in = smem + kOffSmemActIn;
-	unsigned char* act_h = smem + kOffSmemActH;
-	float2* xch = reinterpret_cast<float2*>(smem + kOffSmemXch);
+	unsigned char* act = smem + kOffSmemAct + team * kActBytes;
+	float2* xch = reinterpret_cast<float2*>(smem + kOffSmemXch) + team * (kParts * kTile);
 	const uint32_t w_addr[5] = {smem_u32(smem + kOffImgW0), smem_u32(smem + kOffImgW1), smem_u32(smem + kOffImgW2),
 	                            smem_u32(smem + kOffImgW3), smem_u32(smem + kOffImgW4)};
 
 	uint32_t phase = 0;
 	bool failed = false;
 	const uint32_t num_tiles = (n + kTile - 1) / kTile;
-	for(uint32_t tile = blockIdx.x; tile < num_tiles && !failed; tile += gridDim.x)
+	// (a team's first tile is gridDim.x after the previous team's, so that few tiles spread over the SMs)
+	for(uint32_t tile = team * gridDim.x + blockIdx.x; tile < num_tiles && !failed; tile += kTeams * gridDim.x)
 	{
 		const uint32_t row = tile * kTile + r;
 		const bool valid = row < n;
@@ -154,15 +180,14 @@ mlp_forward_kernel(const unsigned char* __restrict__ image, const float* __restr
 			f[i] = valid ? __ldg(features + static_cast<size_t>(row) * 8 + i) : -1.0f;
 		}
 
-		// One MMA chain (k_steps x K = 16) from A buffer a_buf against weights w_base starting at
+		// One MMA chain (k_steps x K = 16) from the team's A buffer against weights w_base starting at
 		// global K-step ks0, committed to the mbarrier; every thread then waits for it.
-		auto run_mma = [&](const unsigned char* a_buf, uint32_t k_steps, uint32_t w_base, uint32_t n_dim,
-		                   uint32_t ks0, bool accumulate) -> bool
+		auto run_mma = [&](uint32_t k_steps, uint32_t w_base, uint32_t n_dim, uint32_t ks0, bool accumulate) -> bool
 		{
 			if(tid == 0)
 			{
 				fence_after_sync();
-				const uint32_t a_base = smem_u32(a_buf);
+				const uint32_t a_base = smem_u32(act);
 				const uint32_t idesc = instr_desc(kTile, n_dim);
 				for(uint32_t ks = 0; ks < k_steps; ++ks)
 				{
@@ -172,10 +197,10 @@ mlp_forward_kernel(const unsigned char* __restrict__ image, const float* __restr
 				}
 				mma_commit(bar);
 			}
-			// one thread polls the barrier; the others wait at the block barrier, which issues no
+			// one thread polls the barrier; the others wait at the team's barrier, which issues no
 			// instructions while the MMAs run
 			const bool ok = tid == 0 ? mbar_wait(bar, phase) : true;
-			if(__syncthreads_or(ok ? 0 : 1))
+			if(team_sync_or(team, !ok))
 			{
 				// the tensor cores did not report back: one more bounded wait for this phase so
 				// that the accumulator is not freed under running MMAs, then give up
@@ -226,14 +251,14 @@ mlp_forward_kernel(const unsigned char* __restrict__ image, const float* __restr
 						g *= ratio;
 						ratio *= 0.36787944117144233f;   // e^-1
 					}
-					store_row8(act_in, r, static_cast<uint32_t>((i - i0) * kBins + c * 8), v);
+					store_row8(act, r, static_cast<uint32_t>((i - i0) * kBins + c * 8), v);
 				}
 			}
 			fence_async_smem();
 			fence_before_sync();
-			__syncthreads();
+			team_sync(team);
 			const uint32_t k_steps = (half == 0 ? kInHalf0 : kInHalf1) / 16;
-			tile_ok = run_mma(act_in, k_steps, w_addr[0], kHidden, half == 0 ? 0u : kInHalf0 / 16, half == 1);
+			tile_ok = run_mma(k_steps, w_addr[0], kHidden, half == 0 ? 0u : kInHalf0 / 16, half == 1);
 		}
 		if(!tile_ok)
 		{
@@ -241,17 +266,15 @@ mlp_forward_kernel(const unsigned char* __restrict__ image, const float* __restr
 			break;
 		}
 
-		// 2./3. H1 (act_h) -> H2 (act_in) -> H3 (act_h) -> H4 (act_in) -> out
+		// 2./3. H1 -> H2 -> H3 -> H4 -> out
 		#pragma unroll 1
 		for(int layer = 0; layer < 5; ++layer)
 		{
 			const bool last = layer == 4;
 			const uint32_t n_dim = last ? kOutPad : kHidden;
-			unsigned char* o_buf = (layer & 1) ? act_in : act_h;
 			if(layer > 0)
 			{
-				const unsigned char* a_buf = (layer & 1) ? act_h : act_in;
-				if(!run_mma(a_buf, kHidden / 16, w_addr[layer], n_dim, 0u, false))
+				if(!run_mma(kHidden / 16, w_addr[layer], n_dim, 0u, false))
 				{
 					failed = true;
 					break;
@@ -275,7 +298,7 @@ mlp_forward_kernel(const unsigned char* __restrict__ image, const float* __restr
 				#pragma unroll
 				for(int c = 0; c < 4; ++c)
 				{
-					store_row8(o_buf, r, c0 + c * 8, acc + c * 8);
+					store_row8(act, r, c0 + c * 8, acc + c * 8);
 				}
 				if(out_acts && valid)
 				{
@@ -323,7 +346,7 @@ mlp_forward_kernel(const unsigned char* __restrict__ image, const float* __restr
 						mx = fmaxf(mx, raw[5 * j]);
 					}
 					xch[part * kTile + r].x = mx;
-					__syncthreads();
+					team_sync(team);
 					mx = fmaxf(xch[r].x, xch[kTile + r].x);
 					float e[4], sum = 0.0f;
 					#pragma unroll
@@ -333,7 +356,7 @@ mlp_forward_kernel(const unsigned char* __restrict__ image, const float* __restr
 						sum += e[j];
 					}
 					xch[part * kTile + r].y = sum;
-					__syncthreads();
+					team_sync(team);
 					sum = xch[r].y + xch[kTile + r].y;
 					if(valid)
 					{
@@ -356,7 +379,7 @@ mlp_forward_kernel(const unsigned char* __restrict__ image, const float* __restr
 			}
 			fence_async_smem();
 			fence_before_sync();
-			__syncthreads();
+			team_sync(team);
 			fence_after_sync();
 		}
 	}
@@ -369,7 +392,7 @@ mlp_forward_kernel(const unsigned char* __restrict__ image, const float* __restr
 	__syncthreads();
 	if(warp == 0)
 	{
-		asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(kTmemCols) : "memory");
+		asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem_base), "r"(kTmemCols) : "memory");
 	}
 }
 
@@ -446,7 +469,7 @@ void launch_forward(const unsigned char* d_image, const float* d_features, uint3
 	}();
 	(void)configured;
 	const uint32_t tiles = (n + kTile - 1) / kTile;
-	const uint32_t grid = std::min<uint32_t>(tiles, 2u * static_cast<uint32_t>(sm_count()));
+	const uint32_t grid = std::min<uint32_t>(tiles, static_cast<uint32_t>(sm_count()));
 	mlp_forward_kernel<<<grid, kThreads, kSmemBytes, s>>>(d_image, d_features, n, d_n, d_out_raw, d_out_mix,
 	                                                     d_out_acts, d_error);
 	PG_CUDA_CHECK(cudaGetLastError());
