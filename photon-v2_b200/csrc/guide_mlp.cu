@@ -34,8 +34,7 @@
 
 #include <cuda_bf16.h>
 
-#include <cstring>
-#include <vector>
+#include <algorithm>
 
 namespace pg
 {
@@ -444,9 +443,45 @@ __global__ void pack_image_kernel(const float* __restrict__ params, unsigned cha
 	}
 }
 
+// Rows as the host has them (raw: features [n][7], then directions [n][3], then weights [n]) -> padded rows.
+__global__ void spread_rows_kernel(const float* __restrict__ raw, uint64_t n, float* __restrict__ features,
+                                   float4* __restrict__ dirw)
+{
+	for(uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < n;
+	    i += gridDim.x * static_cast<uint64_t>(blockDim.x))
+	{
+		const float* f = raw + i * kInputs;
+		float4* dst = reinterpret_cast<float4*>(features + i * 8);
+		dst[0] = make_float4(f[0], f[1], f[2], f[3]);
+		dst[1] = make_float4(f[4], f[5], f[6], 0.0f);
+		if(dirw)
+		{
+			const float* d = raw + n * kInputs + i * 3;
+			dirw[i] = make_float4(d[0], d[1], d[2], raw[n * (kInputs + 3) + i]);
+		}
+	}
+}
+
 }// end anonymous namespace
 
 int image_bytes() { return kImageBytes; }
+
+void upload_rows(const float* features, const float* dirs, const float* weights, uint64_t n, float* d_features,
+                 float4* d_dirw, cudaStream_t s)
+{
+	ScratchBuffer<float> raw(n * (d_dirw ? kInputs + 4 : kInputs));
+	float* at = raw.get();
+	PG_CUDA_CHECK(cudaMemcpyAsync(at, features, n * kInputs * sizeof(float), cudaMemcpyHostToDevice, s));
+	if(d_dirw)
+	{
+		at += n * kInputs;
+		PG_CUDA_CHECK(cudaMemcpyAsync(at, dirs, n * 3 * sizeof(float), cudaMemcpyHostToDevice, s));
+		PG_CUDA_CHECK(cudaMemcpyAsync(at + n * 3, weights, n * sizeof(float), cudaMemcpyHostToDevice, s));
+	}
+	const uint64_t blocks = std::min<uint64_t>((n + 255u) / 256u, 8u * static_cast<uint64_t>(sm_count()));
+	spread_rows_kernel<<<static_cast<unsigned>(blocks), 256, 0, s>>>(raw.get(), n, d_features, d_dirw);
+	PG_CUDA_CHECK(cudaGetLastError());
+}
 
 void pack_image(const float* d_params, unsigned char* d_image, cudaStream_t s)
 {
@@ -502,21 +537,15 @@ void forward_on_host(const char* what, const float* params, const float* feature
 		return;
 	}
 	cudaStream_t s = library_stream();
-	DeviceBuffer<float> d_params(guide::kNumParams);
-	DeviceBuffer<unsigned char> d_image(guide::image_bytes());
-	DeviceBuffer<float> d_feat(n * 8);
-	DeviceBuffer<float> d_raw(out_raw ? n * guide::kOut : 0);
-	DeviceBuffer<float> d_mix(out_mix ? n * guide::kMixFloats : 0);
-	DeviceBuffer<uint32_t> d_err(1);
+	ScratchBuffer<float> d_params(guide::kNumParams);
+	ScratchBuffer<unsigned char> d_image(guide::image_bytes());
+	ScratchBuffer<float> d_feat(n * 8);
+	ScratchBuffer<float> d_raw(out_raw ? n * guide::kOut : 0);
+	ScratchBuffer<float> d_mix(out_mix ? n * guide::kMixFloats : 0);
+	ScratchBuffer<uint32_t> d_err(1);
 	PG_CUDA_CHECK(cudaMemsetAsync(d_err.get(), 0, sizeof(uint32_t), s));
 	PG_CUDA_CHECK(cudaMemcpyAsync(d_params.get(), params, d_params.bytes(), cudaMemcpyHostToDevice, s));
-	// features: host [n][7] -> device [n][8]
-	std::vector<float> feat(n * 8, 0.0f);
-	for(uint64_t i = 0; i < n; ++i)
-	{
-		std::memcpy(&feat[i * 8], features + i * guide::kInputs, sizeof(float) * guide::kInputs);
-	}
-	PG_CUDA_CHECK(cudaMemcpyAsync(d_feat.get(), feat.data(), d_feat.bytes(), cudaMemcpyHostToDevice, s));
+	guide::upload_rows(features, nullptr, nullptr, n, d_feat.get(), nullptr, s);
 	guide::pack_image(d_params.get(), d_image.get(), s);
 	guide::launch_forward(d_image.get(), d_feat.get(), static_cast<uint32_t>(n), out_raw ? d_raw.get() : nullptr,
 	                      nullptr, d_err.get(), s, nullptr, out_mix ? d_mix.get() : nullptr);

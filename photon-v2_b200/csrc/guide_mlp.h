@@ -17,6 +17,12 @@ int image_bytes();
 // FP32 parameters (kNumParams, packed order of guide.cuh) -> weight image.
 void pack_image(const float* d_params, unsigned char* d_image, cudaStream_t s);
 
+// Host arrays as the entry points take them -- features [n][7], and for training directions [n][3]
+// and weights [n] (d_dirw null: neither) -- to the layouts the kernels read, d_features [n][8] and
+// d_dirw [n]. The rows are copied as they are and spread out on the device.
+void upload_rows(const float* features, const float* dirs, const float* weights, uint64_t n, float* d_features,
+                 float4* d_dirw, cudaStream_t s);
+
 // Forward pass of n queries. d_features: [n][8] FP32 (7 used). d_out_raw: [n][40] FP32 raw
 // outputs (decode() turns them into a mixture). d_out_acts (optional): [n][4][64] BF16 post-ReLU
 // hidden activations, for training. Errors are OR-ed into *d_error (PG_DEV_ERR_GUIDE_WAIT).

@@ -752,26 +752,6 @@ void launch_adam(float* d_params, float* d_grads, float* d_m, float* d_v, uint32
 
 using namespace pg;
 
-namespace
-{
-
-// Host [n][7] features, [n][3] directions, [n] weights -> device [n][8] and [n] float4.
-void upload_batch(const float* features, const float* dirs, const float* weights, uint64_t n,
-                  DeviceBuffer<float>& d_feat, DeviceBuffer<float4>& d_dirw, cudaStream_t s)
-{
-	std::vector<float> feat(n * 8, 0.0f);
-	std::vector<float4> dw(n);
-	for(uint64_t i = 0; i < n; ++i)
-	{
-		std::memcpy(&feat[i * 8], features + i * guide::kInputs, sizeof(float) * guide::kInputs);
-		dw[i] = make_float4(dirs[3 * i], dirs[3 * i + 1], dirs[3 * i + 2], weights[i]);
-	}
-	PG_CUDA_CHECK(cudaMemcpyAsync(d_feat.get(), feat.data(), d_feat.bytes(), cudaMemcpyHostToDevice, s));
-	PG_CUDA_CHECK(cudaMemcpyAsync(d_dirw.get(), dw.data(), d_dirw.bytes(), cudaMemcpyHostToDevice, s));
-}
-
-}// end anonymous namespace
-
 extern "C" {
 
 int pgpu_guide_gradients(const float* params, const float* features, const float* dirs, const float* weights,
@@ -795,17 +775,17 @@ int pgpu_guide_gradients_ex(const float* params, const float* features, const fl
 		}
 		require_device();
 		cudaStream_t s = library_stream();
-		DeviceBuffer<float> d_params(guide::kNumParams), d_grads(guide::kNumParams);
-		DeviceBuffer<unsigned char> d_image(guide::image_bytes());
-		DeviceBuffer<float> d_feat(n * 8), d_raw(n * guide::kOut), d_scalars(2);
-		DeviceBuffer<float4> d_dirw(n);
-		DeviceBuffer<__nv_bfloat16> d_acts(n * guide::kHiddenLayers * guide::kHidden);
-		DeviceBuffer<uint32_t> d_err(1);
+		ScratchBuffer<float> d_params(guide::kNumParams), d_grads(guide::kNumParams);
+		ScratchBuffer<unsigned char> d_image(guide::image_bytes());
+		ScratchBuffer<float> d_feat(n * 8), d_raw(n * guide::kOut), d_scalars(2);
+		ScratchBuffer<float4> d_dirw(n);
+		ScratchBuffer<__nv_bfloat16> d_acts(n * guide::kHiddenLayers * guide::kHidden);
+		ScratchBuffer<uint32_t> d_err(1);
 		PG_CUDA_CHECK(cudaMemsetAsync(d_err.get(), 0, sizeof(uint32_t), s));
 		PG_CUDA_CHECK(cudaMemsetAsync(d_grads.get(), 0, d_grads.bytes(), s));
 		PG_CUDA_CHECK(cudaMemsetAsync(d_scalars.get(), 0, d_scalars.bytes(), s));
 		PG_CUDA_CHECK(cudaMemcpyAsync(d_params.get(), params, d_params.bytes(), cudaMemcpyHostToDevice, s));
-		upload_batch(features, dirs, weights, n, d_feat, d_dirw, s);
+		guide::upload_rows(features, dirs, weights, n, d_feat.get(), d_dirw.get(), s);
 		guide::pack_image(d_params.get(), d_image.get(), s);
 		guide::launch_gradients(d_params.get(), d_image.get(), d_feat.get(), d_dirw.get(), static_cast<uint32_t>(n),
 		                        d_raw.get(), d_acts.get(), d_grads.get(), d_scalars.get(), d_scalars.get() + 1,
@@ -840,13 +820,13 @@ int pgpu_guide_train(float* params, const float* features, const float* dirs, co
 		require_device();
 		cudaStream_t s = library_stream();
 		const uint32_t b = static_cast<uint32_t>(std::min<uint64_t>(batch, n));
-		DeviceBuffer<float> d_params(guide::kNumParams), d_grads(guide::kNumParams), d_m(guide::kNumParams),
+		ScratchBuffer<float> d_params(guide::kNumParams), d_grads(guide::kNumParams), d_m(guide::kNumParams),
 			d_v(guide::kNumParams);
-		DeviceBuffer<unsigned char> d_image(guide::image_bytes());
-		DeviceBuffer<float> d_feat(n * 8), d_raw(b * guide::kOut), d_scalars(2 * steps);
-		DeviceBuffer<float4> d_dirw(n);
-		DeviceBuffer<__nv_bfloat16> d_acts(static_cast<size_t>(b) * guide::kHiddenLayers * guide::kHidden);
-		DeviceBuffer<uint32_t> d_err(1), d_step(1);
+		ScratchBuffer<unsigned char> d_image(guide::image_bytes());
+		ScratchBuffer<float> d_feat(n * 8), d_raw(static_cast<std::size_t>(b) * guide::kOut), d_scalars(2 * static_cast<std::size_t>(steps));
+		ScratchBuffer<float4> d_dirw(n);
+		ScratchBuffer<__nv_bfloat16> d_acts(static_cast<size_t>(b) * guide::kHiddenLayers * guide::kHidden);
+		ScratchBuffer<uint32_t> d_err(1), d_step(1);
 		PG_CUDA_CHECK(cudaMemsetAsync(d_err.get(), 0, sizeof(uint32_t), s));
 		PG_CUDA_CHECK(cudaMemsetAsync(d_step.get(), 0, sizeof(uint32_t), s));
 		PG_CUDA_CHECK(cudaMemsetAsync(d_grads.get(), 0, d_grads.bytes(), s));
@@ -854,7 +834,7 @@ int pgpu_guide_train(float* params, const float* features, const float* dirs, co
 		PG_CUDA_CHECK(cudaMemsetAsync(d_v.get(), 0, d_v.bytes(), s));
 		PG_CUDA_CHECK(cudaMemsetAsync(d_scalars.get(), 0, d_scalars.bytes(), s));
 		PG_CUDA_CHECK(cudaMemcpyAsync(d_params.get(), params, d_params.bytes(), cudaMemcpyHostToDevice, s));
-		upload_batch(features, dirs, weights, n, d_feat, d_dirw, s);
+		guide::upload_rows(features, dirs, weights, n, d_feat.get(), d_dirw.get(), s);
 		for(uint32_t step = 0; step < steps; ++step)
 		{
 			const uint32_t first = static_cast<uint32_t>((static_cast<uint64_t>(step) * b) % n);
@@ -865,7 +845,7 @@ int pgpu_guide_train(float* params, const float* features, const float* dirs, co
 			                        d_scalars.get() + 2 * step, d_scalars.get() + 2 * step + 1, d_err.get(), s);
 			guide::launch_adam(d_params.get(), d_grads.get(), d_m.get(), d_v.get(), d_step.get(), lr, s);
 		}
-		std::vector<float> scalars(2 * steps);
+		std::vector<float> scalars(2 * static_cast<std::size_t>(steps));
 		uint32_t err = 0;
 		PG_CUDA_CHECK(cudaMemcpyAsync(params, d_params.get(), d_params.bytes(), cudaMemcpyDeviceToHost, s));
 		PG_CUDA_CHECK(cudaMemcpyAsync(scalars.data(), d_scalars.get(), d_scalars.bytes(), cudaMemcpyDeviceToHost, s));

@@ -91,7 +91,7 @@ extern "C" int pgpu_bsdf_eval(const float* cases, const float* normals, uint64_t
 			return;
 		}
 		cudaStream_t s = library_stream();
-		DeviceBuffer<float> d_cases(n * kCaseIn), d_normals(n * 6), d_out(n * kCaseOut);
+		ScratchBuffer<float> d_cases(n * kCaseIn), d_normals(n * 6), d_out(n * kCaseOut);
 		PG_CUDA_CHECK(cudaMemcpyAsync(d_cases.get(), cases, d_cases.bytes(), cudaMemcpyHostToDevice, s));
 		PG_CUDA_CHECK(cudaMemcpyAsync(d_normals.get(), normals, d_normals.bytes(), cudaMemcpyHostToDevice, s));
 		bsdf_cases_kernel<<<static_cast<unsigned>((n + 127) / 128), 128, 0, s>>>(

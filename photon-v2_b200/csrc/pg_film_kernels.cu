@@ -55,11 +55,11 @@ extern "C" int pgpu_film_splat(uint32_t filter, uint32_t width, uint32_t height,
 		}
 		require_device();
 		cudaStream_t s = library_stream();
-		DeviceBuffer<double> d_sums(static_cast<std::size_t>(width) * height * kFilmChannels);
+		ScratchBuffer<double> d_sums(static_cast<std::size_t>(width) * height * kFilmChannels);
 		PG_CUDA_CHECK(cudaMemsetAsync(d_sums.get(), 0, d_sums.bytes(), s));
 		if(n > 0)
 		{
-			DeviceBuffer<float> d_samples(n * kSampleFloats);
+			ScratchBuffer<float> d_samples(n * kSampleFloats);
 			PG_CUDA_CHECK(cudaMemcpyAsync(d_samples.get(), samples, d_samples.bytes(), cudaMemcpyHostToDevice, s));
 			const FilmView f = make_film_view(d_sums.get(), width, height, filter);
 			film_splat_kernel<<<static_cast<unsigned>((n + 127) / 128), 128, 0, s>>>(f, d_samples.get(), n);

@@ -20,6 +20,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <type_traits>
 
 namespace cg = cooperative_groups;
 
@@ -1708,31 +1709,50 @@ void RenderScene::ensure_capacity(uint32_t capacity, uint32_t grid)
 	}
 	++m_buffer_generation;
 	capacity = std::max(capacity, m_capacity);
-	for(int b = 0; b < 2; ++b)
+	// the slots the blocks of one residue visit in classify_kernel's grid-stride loop
+	const uint32_t rounds = (capacity + grid * kShadeBlock - 1u) / (grid * kShadeBlock);
+	m_order_list = (grid + kClassLists - 1u) / kClassLists * rounds * kShadeBlock;
+	// One allocation for the whole pool (0.8 GB at 2^21 slots): about thirty of them, one per array,
+	// took most of a new scene's first render of a small image. Two rounds: sizes, then addresses.
+	std::size_t total = 0;
+	for(int round = 0; round < 2; ++round)
 	{
-		m_path[b].resize(capacity);
-		m_meta[b].resize(capacity);
-		m_thr[b].resize(capacity);
-		m_rad[b].resize(capacity);
-		m_prev[b].resize(capacity);
-		m_ro[b].resize(capacity);
-		m_rd[b].resize(capacity);
-	}
-	m_hits.resize(capacity);
-	for(int b = 0; b < 2; ++b)
-	{
-		m_so[b].resize(capacity);
-		m_sd[b].resize(capacity);
-		m_sc[b].resize(capacity);
-		m_sr[b].resize(capacity);
-	}
-	m_req_single.resize(capacity);
-	m_req_mutual.resize(capacity);
-	{
-		// the slots the blocks of one residue visit in classify_kernel's grid-stride loop
-		const uint32_t rounds = (capacity + grid * kShadeBlock - 1u) / (grid * kShadeBlock);
-		m_order_list = (grid + kClassLists - 1u) / kClassLists * rounds * kShadeBlock;
-		m_order.resize(static_cast<size_t>(kOrderLists) * m_order_list);
+		unsigned char* const base = round == 0 ? nullptr : m_pool.get();
+		std::size_t at = 0;
+		auto carve = [&](auto& span, std::size_t n)
+		{
+			using T = std::remove_pointer_t<decltype(span.get())>;
+			if(base)
+			{
+				span.set(base + at, n);
+			}
+			at += (n * sizeof(T) + 255u) / 256u * 256u;
+		};
+		for(int b = 0; b < 2; ++b)
+		{
+			carve(m_path[b], capacity);
+			carve(m_meta[b], capacity);
+			carve(m_thr[b], capacity);
+			carve(m_rad[b], capacity);
+			carve(m_prev[b], capacity);
+			carve(m_ro[b], capacity);
+			carve(m_rd[b], capacity);
+			carve(m_so[b], capacity);
+			carve(m_sd[b], capacity);
+			carve(m_sc[b], capacity);
+			carve(m_sr[b], capacity);
+		}
+		carve(m_hits, capacity);
+		carve(m_req_single, capacity);
+		carve(m_req_mutual, capacity);
+		carve(m_order, static_cast<std::size_t>(kOrderLists) * m_order_list);
+		if(round == 0)
+		{
+			total = at;
+			m_capacity = 0;      // the old pool goes first
+			m_pool.release();
+			m_pool.resize(total);
+		}
 	}
 	m_capacity = capacity;
 	m_order_grid = grid;

@@ -459,13 +459,15 @@ private:
 	uint32_t m_bvh_builder = 0;
 	std::vector<uint32_t> m_material_types;   // per material (fingerprint)
 	uint32_t m_shade_kinds = 0;               // bit per shading kernel the materials need besides the matte one
-	DeviceBuffer<uint32_t> m_path[2], m_meta[2];
-	DeviceBuffer<float4>   m_thr[2], m_rad[2], m_prev[2], m_ro[2], m_rd[2];
-	DeviceBuffer<uint2>    m_hits;
-	DeviceBuffer<float4>   m_so[2], m_sd[2], m_sc[2];   // shadow queues, one per iteration parity
-	DeviceBuffer<float2>   m_sr[2];
-	DeviceBuffer<uint32_t> m_req_single, m_req_mutual;
-	DeviceBuffer<uint32_t> m_order;   // shading order: kOrderLists lists of m_order_list slots
+	// the path pool: one allocation, carved by ensure_capacity
+	DeviceBuffer<unsigned char> m_pool;
+	DeviceSpan<uint32_t> m_path[2], m_meta[2];
+	DeviceSpan<float4>   m_thr[2], m_rad[2], m_prev[2], m_ro[2], m_rd[2];
+	DeviceSpan<uint2>    m_hits;
+	DeviceSpan<float4>   m_so[2], m_sd[2], m_sc[2];   // shadow queues, one per iteration parity
+	DeviceSpan<float2>   m_sr[2];
+	DeviceSpan<uint32_t> m_req_single, m_req_mutual;
+	DeviceSpan<uint32_t> m_order;   // shading order: kOrderLists lists of m_order_list slots
 	DeviceBuffer<float4>   m_samples; // 4 x 4 filters: radiance of every path of a pass
 	DeviceBuffer<uint32_t> m_inflight;   // previews: paths in flight per pixel
 	DeviceBuffer<uint32_t> m_ssid[2];    // multi-scene renders: scene of each NEE record

@@ -62,6 +62,85 @@ cudaStream_t library_stream()
 	return streams[dev];
 }
 
+namespace
+{
+
+std::mutex g_scratch_mutex;
+cudaMemPool_t g_scratch_pools[kMaxDevices] = {};
+
+cudaMemPool_t scratch_pool()
+{
+	const int dev = current_device();
+	std::lock_guard<std::mutex> lock(g_scratch_mutex);
+	if(!g_scratch_pools[dev])
+	{
+		cudaMemPoolProps props{};
+		props.allocType = cudaMemAllocationTypePinned;
+		props.location.type = cudaMemLocationTypeDevice;
+		props.location.id = dev;
+		cudaMemPool_t pool = nullptr;
+		PG_CUDA_CHECK(cudaMemPoolCreate(&pool, &props));
+		uint64_t kept = kScratchKept;
+		const cudaError_t status = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &kept);
+		if(status != cudaSuccess)
+		{
+			cudaMemPoolDestroy(pool);
+			cudaGetLastError();
+			throw Error(PG_ERR_CUDA, std::string("cudaMemPoolSetAttribute: ") + cudaGetErrorString(status));
+		}
+		g_scratch_pools[dev] = pool;
+	}
+	return g_scratch_pools[dev];
+}
+
+}// end anonymous namespace
+
+void* scratch_alloc(std::size_t bytes)
+{
+	void* p = nullptr;
+	PG_CUDA_CHECK(cudaMallocFromPoolAsync(&p, bytes, scratch_pool(), library_stream()));
+	return p;
+}
+
+void scratch_free(void* p) noexcept
+{
+	// (the stream exists: the allocation was made on it)
+	try
+	{
+		cudaFreeAsync(p, library_stream());
+	}
+	catch(...)
+	{
+	}
+}
+
+void trim_scratch()
+{
+	std::lock_guard<std::mutex> lock(g_scratch_mutex);
+	for(cudaMemPool_t pool : g_scratch_pools)
+	{
+		if(pool)
+		{
+			cudaMemPoolTrimTo(pool, 0);
+		}
+	}
+}
+
+unsigned char* pinned_stage()
+{
+	struct Stage
+	{
+		void* p = nullptr;
+		~Stage() { if(p) { cudaFreeHost(p); } }
+	};
+	static thread_local Stage stage;
+	if(!stage.p)
+	{
+		PG_CUDA_CHECK(cudaHostAlloc(&stage.p, kPinnedStage, cudaHostAllocPortable));
+	}
+	return static_cast<unsigned char*>(stage.p);
+}
+
 void check_same_device(int owner_device, int current, const char* what)
 {
 	if(current != owner_device)

@@ -119,6 +119,12 @@ public:
 		return true;
 	}
 
+	bool empty()
+	{
+		std::lock_guard<std::mutex> lock(m_mutex);
+		return m_items.empty();
+	}
+
 private:
 	std::mutex m_mutex;
 	uint64_t m_next = 0;
@@ -194,6 +200,53 @@ private:
 	T* m_ptr = nullptr;
 	std::size_t m_size = 0;
 };
+
+// A view of a part of a DeviceBuffer (render pools carve theirs out of one allocation).
+template<typename T>
+class DeviceSpan
+{
+public:
+	void set(void* p, std::size_t n) { m_ptr = static_cast<T*>(p); m_size = n; }
+	T* get() const { return m_ptr; }
+	std::size_t size() const { return m_size; }
+	std::size_t bytes() const { return m_size * sizeof(T); }
+
+private:
+	T* m_ptr = nullptr;
+	std::size_t m_size = 0;
+};
+
+// Device memory for one call, in stream order on the library stream: taken from the device's scratch
+// pool and handed back when the buffer's scope ends, after the work queued by then. cudaMalloc and
+// cudaFree, which wait for the device, cost a query of 1,000 rays more than its kernels. The pool
+// keeps at most kScratchKept bytes between calls (trim_scratch gives those back too) and may be
+// used from several threads.
+constexpr std::size_t kScratchKept = std::size_t(256) << 20;
+void* scratch_alloc(std::size_t bytes);
+void scratch_free(void* p) noexcept;
+void trim_scratch();
+
+template<typename T>
+class ScratchBuffer
+{
+public:
+	explicit ScratchBuffer(std::size_t n) : m_ptr(n ? static_cast<T*>(scratch_alloc(n * sizeof(T))) : nullptr), m_size(n) {}
+	~ScratchBuffer() { if(m_ptr) { scratch_free(m_ptr); } }
+	ScratchBuffer(const ScratchBuffer&) = delete;
+	ScratchBuffer& operator = (const ScratchBuffer&) = delete;
+	T* get() const { return m_ptr; }
+	std::size_t size() const { return m_size; }
+	std::size_t bytes() const { return m_size * sizeof(T); }
+
+private:
+	T* m_ptr;
+	std::size_t m_size;
+};
+
+// Page-locked host memory of the calling thread for small results (one copy instead of one per output
+// array, at the latency of the link). Larger results go straight to the caller's arrays.
+constexpr std::size_t kPinnedStage = std::size_t(256) << 10;
+unsigned char* pinned_stage();
 
 // Number of SMs of the current device (grid sizing).
 int sm_count();

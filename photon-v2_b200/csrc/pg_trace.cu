@@ -7,6 +7,7 @@
 #include "../../include/photon_gpu.h"
 
 #include <algorithm>
+#include <cstring>
 #include <map>
 #include <mutex>
 #include <string>
@@ -192,16 +193,23 @@ std::shared_ptr<Geometry> get_geometry(uint64_t id)
 	return g;
 }
 
-void check_device_error(Geometry& g, cudaStream_t s)
+// Turns the geometry's error flags, read after the work, into an exception (and clears them).
+void raise_device_error(Geometry& g, uint32_t flags, cudaStream_t s)
 {
-	uint32_t flags = 0;
-	PG_CUDA_CHECK(cudaMemcpyAsync(&flags, g.error.get(), sizeof(flags), cudaMemcpyDeviceToHost, s));
-	PG_CUDA_CHECK(cudaStreamSynchronize(s));
 	if(flags & PG_DEV_ERR_STACK)
 	{
 		PG_CUDA_CHECK(cudaMemsetAsync(g.error.get(), 0, sizeof(uint32_t), s));
 		throw Error(PG_ERR_STACK_OVERFLOW, "BVH traversal stack overflow");
 	}
+}
+
+void check_device_error(Geometry& g, cudaStream_t s)
+{
+	uint32_t flags = 0;
+	PG_CUDA_CHECK(cudaMemcpyAsync(pinned_stage(), g.error.get(), sizeof(flags), cudaMemcpyDeviceToHost, s));
+	PG_CUDA_CHECK(cudaStreamSynchronize(s));
+	std::memcpy(&flags, pinned_stage(), sizeof(flags));
+	raise_device_error(g, flags, s);
 }
 
 // An unoccluded NEE contribution (shadow record i): to the owning path's radiance (slot in the
@@ -487,6 +495,10 @@ int pgpu_geometry_destroy(uint64_t id)
 		{
 			throw Error(PG_ERR_NOT_FOUND, "unknown geometry id " + std::to_string(id));
 		}
+		if(geometry_registry().empty())
+		{
+			trim_scratch();
+		}
 	});
 }
 
@@ -518,26 +530,41 @@ int pgpu_trace_closest(uint64_t id, const float* rays, uint64_t n,
 			return;
 		}
 		cudaStream_t s = library_stream();
-		DeviceBuffer<float> d_rays(n * 8);
-		DeviceBuffer<HitRecord> d_hits(n);
-		DeviceBuffer<int32_t> d_prim(n);
-		DeviceBuffer<float> d_t(n), d_bary(3 * n);
+		ScratchBuffer<float> d_rays(n * 8);
+		ScratchBuffer<HitRecord> d_hits(n);
+		// prim, t and barycentrics of all rays, one after the other, then the error flags
+		ScratchBuffer<uint32_t> d_out(5 * n + 1);
+		uint32_t* const d_prim = d_out.get();
+		uint32_t* const d_t = d_prim + n;
+		uint32_t* const d_bary = d_t + n;
+		uint32_t* const d_flags = d_bary + 3 * n;
 		PG_CUDA_CHECK(cudaMemcpyAsync(d_rays.get(), rays, d_rays.bytes(), cudaMemcpyHostToDevice, s));
 		launch_trace_closest(*g, d_rays.get(), n, d_hits.get(), s);
 		resolve_hits_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, s>>>(
 			g->tris.get(), reinterpret_cast<const float4*>(d_rays.get()), d_hits.get(), n,
-			d_prim.get(), d_t.get(), d_bary.get());
+			reinterpret_cast<int32_t*>(d_prim), reinterpret_cast<float*>(d_t), reinterpret_cast<float*>(d_bary));
 		PG_CUDA_CHECK(cudaGetLastError());
-		std::vector<int32_t> prim(n);
-		std::vector<float> t(n), bary(3 * n);
-		PG_CUDA_CHECK(cudaMemcpyAsync(prim.data(), d_prim.get(), d_prim.bytes(), cudaMemcpyDeviceToHost, s));
-		PG_CUDA_CHECK(cudaMemcpyAsync(t.data(), d_t.get(), d_t.bytes(), cudaMemcpyDeviceToHost, s));
-		PG_CUDA_CHECK(cudaMemcpyAsync(bary.data(), d_bary.get(), d_bary.bytes(), cudaMemcpyDeviceToHost, s));
-		PG_CUDA_CHECK(cudaStreamSynchronize(s));
-		check_device_error(*g, s);
-		if(out_prim) { std::copy(prim.begin(), prim.end(), out_prim); }
-		if(out_t) { std::copy(t.begin(), t.end(), out_t); }
-		if(out_bary) { std::copy(bary.begin(), bary.end(), out_bary); }
+		PG_CUDA_CHECK(cudaMemcpyAsync(d_flags, g->error.get(), sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
+		uint32_t flags = 0;
+		if(d_out.bytes() <= kPinnedStage)
+		{
+			const unsigned char* h = pinned_stage();
+			PG_CUDA_CHECK(cudaMemcpyAsync(pinned_stage(), d_out.get(), d_out.bytes(), cudaMemcpyDeviceToHost, s));
+			PG_CUDA_CHECK(cudaStreamSynchronize(s));
+			if(out_prim) { std::memcpy(out_prim, h, 4 * n); }
+			if(out_t) { std::memcpy(out_t, h + 4 * n, 4 * n); }
+			if(out_bary) { std::memcpy(out_bary, h + 8 * n, 12 * n); }
+			std::memcpy(&flags, h + 20 * n, sizeof(flags));
+		}
+		else
+		{
+			if(out_prim) { PG_CUDA_CHECK(cudaMemcpyAsync(out_prim, d_prim, 4 * n, cudaMemcpyDeviceToHost, s)); }
+			if(out_t) { PG_CUDA_CHECK(cudaMemcpyAsync(out_t, d_t, 4 * n, cudaMemcpyDeviceToHost, s)); }
+			if(out_bary) { PG_CUDA_CHECK(cudaMemcpyAsync(out_bary, d_bary, 12 * n, cudaMemcpyDeviceToHost, s)); }
+			PG_CUDA_CHECK(cudaMemcpyAsync(&flags, d_flags, sizeof(flags), cudaMemcpyDeviceToHost, s));
+			PG_CUDA_CHECK(cudaStreamSynchronize(s));
+		}
+		raise_device_error(*g, flags, s);
 	});
 }
 
@@ -555,13 +582,27 @@ int pgpu_trace_any(uint64_t id, const float* rays, uint64_t n, int32_t* out_occl
 			return;
 		}
 		cudaStream_t s = library_stream();
-		DeviceBuffer<float> d_rays(n * 8);
-		DeviceBuffer<int32_t> d_occ(n);
+		ScratchBuffer<float> d_rays(n * 8);
+		ScratchBuffer<int32_t> d_occ(n + 1);   // the answers, then the error flags
 		PG_CUDA_CHECK(cudaMemcpyAsync(d_rays.get(), rays, d_rays.bytes(), cudaMemcpyHostToDevice, s));
 		launch_trace_any(*g, d_rays.get(), n, d_occ.get(), s);
-		PG_CUDA_CHECK(cudaMemcpyAsync(out_occluded, d_occ.get(), d_occ.bytes(), cudaMemcpyDeviceToHost, s));
-		PG_CUDA_CHECK(cudaStreamSynchronize(s));
-		check_device_error(*g, s);
+		PG_CUDA_CHECK(cudaMemcpyAsync(d_occ.get() + n, g->error.get(), sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
+		uint32_t flags = 0;
+		if(d_occ.bytes() <= kPinnedStage)
+		{
+			const unsigned char* h = pinned_stage();
+			PG_CUDA_CHECK(cudaMemcpyAsync(pinned_stage(), d_occ.get(), d_occ.bytes(), cudaMemcpyDeviceToHost, s));
+			PG_CUDA_CHECK(cudaStreamSynchronize(s));
+			std::memcpy(out_occluded, h, 4 * n);
+			std::memcpy(&flags, h + 4 * n, sizeof(flags));
+		}
+		else
+		{
+			PG_CUDA_CHECK(cudaMemcpyAsync(out_occluded, d_occ.get(), 4 * n, cudaMemcpyDeviceToHost, s));
+			PG_CUDA_CHECK(cudaMemcpyAsync(&flags, d_occ.get() + n, sizeof(flags), cudaMemcpyDeviceToHost, s));
+			PG_CUDA_CHECK(cudaStreamSynchronize(s));
+		}
+		raise_device_error(*g, flags, s);
 	});
 }
 
@@ -571,6 +612,12 @@ int pgpu_trace_closest_device(uint64_t id, const float* d_rays, uint64_t n, void
 	{
 		auto g = get_geometry(id);
 		cudaStream_t s = library_stream();
+		if(!out_ms)
+		{
+			launch_trace_closest(*g, d_rays, n, d_hits, s);
+			check_device_error(*g, s);   // (waits for the launch)
+			return;
+		}
 		ScopedEvent e0, e1;
 		PG_CUDA_CHECK(cudaEventRecord(e0.get(), s));
 		launch_trace_closest(*g, d_rays, n, d_hits, s);
@@ -579,7 +626,7 @@ int pgpu_trace_closest_device(uint64_t id, const float* d_rays, uint64_t n, void
 		float ms = 0.0f;
 		PG_CUDA_CHECK(cudaEventElapsedTime(&ms, e0.get(), e1.get()));
 		check_device_error(*g, s);
-		if(out_ms) { *out_ms = ms; }
+		*out_ms = ms;
 	});
 }
 
@@ -589,6 +636,12 @@ int pgpu_trace_any_device(uint64_t id, const float* d_rays, uint64_t n, int32_t*
 	{
 		auto g = get_geometry(id);
 		cudaStream_t s = library_stream();
+		if(!out_ms)
+		{
+			launch_trace_any(*g, d_rays, n, d_occluded, s);
+			check_device_error(*g, s);   // (waits for the launch)
+			return;
+		}
 		ScopedEvent e0, e1;
 		PG_CUDA_CHECK(cudaEventRecord(e0.get(), s));
 		launch_trace_any(*g, d_rays, n, d_occluded, s);
@@ -597,7 +650,7 @@ int pgpu_trace_any_device(uint64_t id, const float* d_rays, uint64_t n, int32_t*
 		float ms = 0.0f;
 		PG_CUDA_CHECK(cudaEventElapsedTime(&ms, e0.get(), e1.get()));
 		check_device_error(*g, s);
-		if(out_ms) { *out_ms = ms; }
+		*out_ms = ms;
 	});
 }
 
@@ -612,8 +665,8 @@ int pgpu_trace_counts(uint64_t id, const float* rays, uint64_t n, int any_hit,
 			throw Error(PG_ERR_INVALID_ARGUMENT, "pgpu_trace_counts: no rays");
 		}
 		cudaStream_t s = library_stream();
-		DeviceBuffer<float> d_rays(n * 8);
-		DeviceBuffer<unsigned long long> d_sums(2);
+		ScratchBuffer<float> d_rays(n * 8);
+		ScratchBuffer<unsigned long long> d_sums(2);
 		PG_CUDA_CHECK(cudaMemcpyAsync(d_rays.get(), rays, d_rays.bytes(), cudaMemcpyHostToDevice, s));
 		PG_CUDA_CHECK(cudaMemsetAsync(d_sums.get(), 0, d_sums.bytes(), s));
 		count_kernel<<<static_cast<unsigned>((n + 127) / 128), 128, 0, s>>>(
@@ -743,8 +796,10 @@ int pgpu_trace_closest_noalloc(uint64_t id, const float* rays, uint64_t n,
 		if(out_prim) { PG_CUDA_CHECK(cudaMemcpyAsync(out_prim, d_prim, n * sizeof(int32_t), cudaMemcpyDeviceToHost, s)); }
 		if(out_t) { PG_CUDA_CHECK(cudaMemcpyAsync(out_t, d_t, n * sizeof(float), cudaMemcpyDeviceToHost, s)); }
 		if(out_bary) { PG_CUDA_CHECK(cudaMemcpyAsync(out_bary, d_bary, 3 * n * sizeof(float), cudaMemcpyDeviceToHost, s)); }
+		uint32_t flags = 0;
+		PG_CUDA_CHECK(cudaMemcpyAsync(&flags, g->error.get(), sizeof(flags), cudaMemcpyDeviceToHost, s));
 		PG_CUDA_CHECK(cudaStreamSynchronize(s));
-		check_device_error(*g, s);
+		raise_device_error(*g, flags, s);
 	});
 }
 
