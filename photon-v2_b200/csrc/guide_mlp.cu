@@ -26,6 +26,7 @@
 // so the descriptor's leading byte offset (between K chunks) is R * 16 and its stride byte offset
 // (between 8-row groups) is 128. Weights are stored transposed (W^T, [out][in]) so that both
 // operands are K-major: D[M x N] = A[M x K] * B[N x K]^T.
+#include "guide_image.cuh"
 #include "guide_mlp.h"
 
 #include "pg_runtime.h"
@@ -54,19 +55,6 @@ constexpr uint32_t kTmemCols = 256;   // power of two >= 64 accumulator columns 
 static_assert(kTeams * kHidden <= static_cast<int>(kTmemCols), "tensor memory");
 static_assert(kParts == 2 && kHidden == 64 && kLobes == 8 && kOut == 40 && kOutPad == 48,
               "the column split below assumes two parts, 64 hidden units and 8 lobes");
-
-// ---- shared-memory image of the weights (also the device-side packed format)
-constexpr int kW0Bytes = kHidden * kIn * 2;         // 28,672
-constexpr int kWhBytes = kHidden * kHidden * 2;     //  8,192
-constexpr int kW4Bytes = kOutPad * kHidden * 2;     //  6,144
-constexpr int kOffImgW0 = 0;
-constexpr int kOffImgW1 = kOffImgW0 + kW0Bytes;
-constexpr int kOffImgW2 = kOffImgW1 + kWhBytes;
-constexpr int kOffImgW3 = kOffImgW2 + kWhBytes;
-constexpr int kOffImgW4 = kOffImgW3 + kWhBytes;
-constexpr int kOffImgBias = kOffImgW4 + kW4Bytes;   // FP32 biases: 4 x 64 + 48
-constexpr int kBiasCount = kHiddenLayers * kHidden + kOutPad;
-constexpr int kImageBytes = kOffImgBias + kBiasCount * 4;   // 60,576
 
 // ---- activation buffer of each team
 // The input layer is fed in two K halves (one-blob inputs 0-3, then 4-6), so that a tile takes 32 KB;

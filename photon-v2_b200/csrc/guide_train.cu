@@ -6,12 +6,13 @@
 // (the KL divergence to the target density up to a constant, Mueller et al. 2019) and its gradient
 // with respect to every parameter, then applies Adam to the FP32 master parameters.
 //
-// Backward pass: one block of 128 threads per 128 samples, thread = sample. Each thread turns its
-// raw outputs into d loss / d raw (the analytic derivative of the vMF mixture's log density) and
+// FP32 backward pass (the cross-check of the tensor-core one below): one block of 128 threads per 128
+// samples, thread = sample. Each thread turns its raw outputs into d loss / d raw (the analytic derivative of the vMF mixture's log density) and
 // back-propagates through the layers with the same BF16-rounded weights the forward pass used.
 // Per layer, the block stages the layer inputs and pre-activation gradients of its 128 samples in
 // shared memory and reduces the weight gradient sum_t x[t][i] dz[t][o] over them (FP32), adding
 // the block's partial to the global gradient with one atomic per weight.
+#include "guide_image.cuh"
 #include "guide_mlp.h"
 
 #include "pg_runtime.h"
@@ -20,7 +21,7 @@
 
 #include <cuda_bf16.h>
 
-#include <cstring>
+#include <algorithm>
 #include <vector>
 
 namespace pg
@@ -308,34 +309,46 @@ backward_kernel(const float* __restrict__ params, const float* __restrict__ feat
 //                           the bias gradient sum_t G_l[t]), N = out_l, K = 128 samples;
 //   dX_l  = G_l W_l^T      MMA M = 128 samples, N = in_l = 64, K = out_l (layers 4..1);
 //   G_l-1 = dX_l where X_l > 0 (the ReLU that produced X_l).
-// The weight gradients stay in tensor memory across all tiles a CTA processes and reach global
-// memory once per CTA. Operands: G_l as sample rows (K = out_l) for dX, and the transposed
+// The weight gradients stay in tensor memory across all tiles a CTA processes; each CTA then writes
+// its sums to a row of its own in `partials`, which the next kernel (Adam, or the reduction of a
+// plain gradient) adds up. Operands: G_l as sample rows (K = out_l) for dX, and the transposed
 // X_l^T / G_l^T (K = samples) for dW, written by each thread for its own sample; the transposed
 // buffers' K-chunk stride carries 16 bytes of padding so that the 8 sample groups a warp writes
 // land in different banks.
+//
+// A step of 16,384 samples is one tile per CTA, a serial chain of six rounds of staging, MMAs and
+// read-back: what counts is the latency of each. Two threads share a sample (part 0: columns 0..31
+// and lobes 0..3, part 1: the rest; thread t and t + 128 on sample t), the next layer's activations
+// are loaded while a round's MMAs run, and the input layer's two halves go through one round. The
+// CTAs' 3.8 M atomics on 29,480 addresses, four bytes each with every lane on a line of its own, had
+// been part of the 145 us that the kernel took at one thread per sample. 32 steps of 16,384 samples through
+// pgpu_guide_train went from 4.87 to 2.30 ms with this kernel and the fused Adam step.
 
 namespace tcb
 {
 
 using namespace tc;
 
-constexpr int kThreads = 128;
+constexpr int kThreads = 256;
+constexpr int kCols = kHidden / 2;                     // hidden columns per thread
 constexpr uint32_t kLboG = kTile * 16u;                // G rows (samples) x K = outputs: 2048
 constexpr uint32_t kLboXT = kTile * 16u + 16u;         // X^T: 128 rows x K = samples, padded: 2064
 constexpr uint32_t kLboGT = kHidden * 16u + 16u;       // G^T: 64 rows x K = samples, padded: 1040
 constexpr uint32_t kLboW = kHidden * 16u;              // W_l: 64 rows (inputs) x K = outputs: 1024
 
 constexpr int kBwHidden = kHidden * kHidden * 2;       // 8,192
+constexpr int kXtBytes = (kTile / 8) * static_cast<int>(kLboXT);          // 33,024
 constexpr int kOffBw = 0;                              // W1, W2, W3, W4 (W4: K = 48)
 constexpr int kOffG = kOffBw + 3 * kBwHidden + kHidden * kOutPad * 2;     // 30,720
-constexpr int kOffXT = kOffG + kTile * kHidden * 2;                       // 47,104
-constexpr int kOffGT = kOffXT + (kTile / 8) * static_cast<int>(kLboXT);   // 80,128
-constexpr int kOffBar = kOffGT + (kTile / 8) * static_cast<int>(kLboGT);  // 96,768
+constexpr int kOffXT = kOffG + kTile * kHidden * 2;                       // 47,104; two buffers
+constexpr int kOffGT = kOffXT + 2 * kXtBytes;                             // 113,152
+constexpr int kOffXch = kOffGT + (kTile / 8) * static_cast<int>(kLboGT);  // 129,792: [part][sample] float3
+constexpr int kOffBar = kOffXch + 2 * kTile * 12;
 constexpr int kOffSlot = kOffBar + 8;
 // More than half an SM's shared memory: one CTA per SM, so that each CTA's 512 TMEM columns are free.
-constexpr int kSmemBytes = 120 * 1024;
-static_assert(kOffSlot + 8 <= kSmemBytes && kSmemBytes <= 227 * 1024, "shared memory");
-static_assert(kOffG % 16 == 0 && kOffXT % 16 == 0 && kOffGT % 16 == 0 && kOffBar % 8 == 0, "alignment");
+constexpr int kSmemBytes = kOffSlot + 8;
+static_assert(kSmemBytes > 114 * 1024 && kSmemBytes <= 227 * 1024, "shared memory");
+static_assert(kOffG % 16 == 0 && kOffXT % 16 == 0 && kOffGT % 16 == 0 && kOffXch % 16 == 0 && kOffBar % 8 == 0, "alignment");
 
 // TMEM columns: the dX accumulator, then the weight gradients of every layer (rows = the layer's
 // inputs, columns = its outputs).
@@ -351,11 +364,78 @@ __device__ __forceinline__ void st_bf16(unsigned char* base, uint32_t off, float
 	*reinterpret_cast<__nv_bfloat16*>(base + off) = __float2bfloat16_rn(v);
 }
 
+__device__ __forceinline__ uint4 pack8(const float* v)
+{
+	return make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+}
+
+// 8 floats to a 32-byte aligned address.
+__device__ __forceinline__ void st_global8(float* p, const float* v)
+{
+	asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+	             :: "l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
+}
+
+// d loss / d raw for this thread's four lobes of a sample (20 values) and, on part 0, the loss term.
+// The two threads of a sample exchange the softmax's maximum and sum and the mixture density through
+// xch. `valid` is the same for both.
+__device__ __forceinline__ void output_gradient_half(const float* raw, V3 d, float scale, bool valid, uint32_t part,
+                                                     float* mine, const float* other, float* g, float* loss_term)
+{
+	float mx = raw[0];
+	#pragma unroll
+	for(int j = 1; j < 4; ++j)
+	{
+		mx = fmaxf(mx, raw[5 * j]);
+	}
+	mine[0] = mx;
+	__syncthreads();
+	mx = fmaxf(mx, other[0]);
+	float w[4], k[4], v[4], cosv[4], sum = 0.0f, q = 0.0f;
+	V3 mu[4];
+	#pragma unroll
+	for(int j = 0; j < 4; ++j)
+	{
+		w[j] = expf(raw[5 * j] - mx);
+		sum += w[j];
+		const V3 m = v3(raw[5 * j + 1], raw[5 * j + 2], raw[5 * j + 3]);
+		const float l2 = dot(m, m);
+		mu[j] = l2 > 1e-20f ? m * (1.0f / sqrtf(l2)) : v3(0.0f, 0.0f, 1.0f);
+		k[j] = fminf(fmaxf(expf(raw[5 * j + 4]), kMinKappa), kMaxKappa);
+		v[j] = vmf_pdf(mu[j], k[j], d);
+		cosv[j] = dot(mu[j], d);
+		q += w[j] * v[j];
+	}
+	mine[1] = sum;
+	mine[2] = q;
+	__syncthreads();
+	sum += other[1];
+	q = fmaxf((q + other[2]) / sum, 1e-30f);
+	*loss_term = part == 0u && valid ? scale * logf(q) : 0.0f;   // scale = -w / total
+	#pragma unroll
+	for(int j = 0; j < 4; ++j)
+	{
+		const float wj = w[j] / sum;
+		const float r = wj * v[j] / q;
+		const float e = expf(-2.0f * k[j]);
+		const float dlogv_dk = 1.0f / k[j] - 2.0f * e / (1.0f - e) + (cosv[j] - 1.0f);
+		const float k_raw = expf(raw[5 * j + 4]);
+		const bool inside = k_raw > kMinKappa && k_raw < kMaxKappa;
+		const V3 m = v3(raw[5 * j + 1], raw[5 * j + 2], raw[5 * j + 3]);
+		const float c = scale * r * k[j] / fmaxf(sqrtf(dot(m, m)), 1e-30f);
+		g[5 * j + 0] = valid ? scale * (r - wj) : 0.0f;
+		g[5 * j + 1] = valid ? c * (d.x - cosv[j] * mu[j].x) : 0.0f;
+		g[5 * j + 2] = valid ? c * (d.y - cosv[j] * mu[j].y) : 0.0f;
+		g[5 * j + 3] = valid ? c * (d.z - cosv[j] * mu[j].z) : 0.0f;
+		g[5 * j + 4] = valid && inside ? scale * r * dlogv_dk * k[j] : 0.0f;
+	}
+}
+
 __global__ void __launch_bounds__(kThreads, 1)
 backward_tc_kernel(const float* __restrict__ params, const float* __restrict__ features,
                    const float4* __restrict__ dirw, const float* __restrict__ raw_out,
                    const __nv_bfloat16* __restrict__ acts, uint32_t n_max, const uint32_t* __restrict__ d_n,
-                   const float* __restrict__ total_weight, float* __restrict__ grads, float* __restrict__ loss,
+                   const float* __restrict__ total_weight, float* __restrict__ partials, float* __restrict__ loss,
                    uint32_t* __restrict__ error)
 {
 	const uint32_t n = d_n ? min(*d_n, n_max) : n_max;
@@ -367,29 +447,29 @@ backward_tc_kernel(const float* __restrict__ params, const float* __restrict__ f
 	extern __shared__ __align__(128) unsigned char smem[];
 	const uint32_t tid = threadIdx.x;
 	const uint32_t warp = tid >> 5;
+	const uint32_t r = tid & (kTile - 1);   // the sample (row) this thread works on
+	const uint32_t part = tid / kTile;      // which half of its columns / lobes
+	const uint32_t c0 = part * kCols;
 
 	// W_1..W_4 as B operands of dX: [64 rows = layer inputs][K = layer outputs], BF16 as the
-	// forward pass rounds them
-	for(uint32_t e = tid; e < 3u * kHidden * kHidden + kHidden * kOutPad; e += kThreads)
+	// forward pass rounds them, 8 outputs at a time
+	for(uint32_t e = tid; e < 3u * kHidden * (kHidden / 8) + kHidden * (kOutPad / 8); e += kThreads)
 	{
-		uint32_t l, i, o, out;
-		if(e < 3u * kHidden * kHidden)
-		{
-			l = 1u + e / (kHidden * kHidden);
-			i = (e % (kHidden * kHidden)) / kHidden;
-			o = e % kHidden;
-			out = kHidden;
-		}
-		else
-		{
-			l = 4u;
-			i = (e - 3u * kHidden * kHidden) / kOutPad;
-			o = (e - 3u * kHidden * kHidden) % kOutPad;
-			out = kOut;
-		}
+		const bool last = e >= 3u * kHidden * (kHidden / 8);
+		const uint32_t f = last ? e - 3u * kHidden * (kHidden / 8) : e % (kHidden * (kHidden / 8));
+		const uint32_t l = last ? 4u : 1u + e / (kHidden * (kHidden / 8));
+		const uint32_t i = last ? f / (kOutPad / 8) : f / (kHidden / 8);
+		const uint32_t o = (last ? f % (kOutPad / 8) : f % (kHidden / 8)) * 8u;
 		const int w_off[5] = {kOffW0, kOffW1, kOffW2, kOffW3, kOffW4};
-		const float w = o < out ? params[w_off[l] + i * out + o] : 0.0f;
-		st_bf16(smem + kOffBw + (l - 1u) * kBwHidden, core_offset_lbo(i, o, kLboW), w);
+		float w[8] = {};
+		if(!last || o < static_cast<uint32_t>(kOut))
+		{
+			const float4* src = reinterpret_cast<const float4*>(params + w_off[l] + i * (last ? kOut : kHidden) + o);
+			const float4 a = __ldg(src), b = __ldg(src + 1);
+			w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
+			w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
+		}
+		*reinterpret_cast<uint4*>(smem + kOffBw + (l - 1u) * kBwHidden + core_offset_lbo(i, o, kLboW)) = pack8(w);
 	}
 	const uint32_t bar = smem_u32(smem + kOffBar);
 	uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kOffSlot);
@@ -409,17 +489,30 @@ backward_tc_kernel(const float* __restrict__ params, const float* __restrict__ f
 	__syncthreads();
 	fence_after_sync();
 	const uint32_t tmem = *tmem_slot;
-	const uint32_t tmem_row = tmem + ((warp * 32u) << 16);
+	const uint32_t tmem_row = tmem + (((warp & 3u) * 32u) << 16);
 
 	unsigned char* gbuf = smem + kOffG;
 	unsigned char* xt = smem + kOffXT;
 	unsigned char* gt = smem + kOffGT;
-	const uint32_t a_g = smem_u32(gbuf), a_xt = smem_u32(xt), a_gt = smem_u32(gt);
+	float* xch = reinterpret_cast<float*>(smem + kOffXch);
+	const uint32_t a_g = smem_u32(gbuf), a_gt = smem_u32(gt);
 
 	uint32_t phase = 0;
 	bool failed = false;
-	// the staged operands -> one dW chain (and, for layers 4..1, one dX chain), committed and awaited
-	auto run = [&](uint32_t col_w, uint32_t n_out, bool acc_w, int dx_layer) -> bool
+	// one dW chain: X^T buffer `x` and G^T into TMEM column col (thread 0)
+	auto weight_chain = [&](const unsigned char* x, uint32_t col, uint32_t n_out, bool accumulate)
+	{
+		const uint32_t a_xt = smem_u32(x);
+		const uint32_t idesc = instr_desc(kTile, n_out);
+		for(uint32_t ks = 0; ks < kTile / 16u; ++ks)
+		{
+			mma_bf16(tmem + col, smem_desc(a_xt + ks * 2u * kLboXT, kLboXT, 128u),
+			         smem_desc(a_gt + ks * 2u * kLboGT, kLboGT, 128u), idesc, (accumulate || ks > 0) ? 1u : 0u);
+		}
+	};
+	// the staged operands -> the round's chains, committed and awaited: layers 4..1 dX (first, the next
+	// round waits for it) and dW; layer 0 the dW of both halves of its inputs
+	auto run = [&](int layer, uint32_t n_out, bool acc_w) -> bool
 	{
 		fence_async_smem();
 		fence_before_sync();
@@ -427,23 +520,21 @@ backward_tc_kernel(const float* __restrict__ params, const float* __restrict__ f
 		if(tid == 0)
 		{
 			fence_after_sync();
-			const uint32_t idesc_w = instr_desc(kTile, n_out);
-			for(uint32_t ks = 0; ks < kTile / 16u; ++ks)
-			{
-				const uint64_t ad = smem_desc(a_xt + ks * 2u * kLboXT, kLboXT, 128u);
-				const uint64_t bd = smem_desc(a_gt + ks * 2u * kLboGT, kLboGT, 128u);
-				mma_bf16(tmem + col_w, ad, bd, idesc_w, (acc_w || ks > 0) ? 1u : 0u);
-			}
-			if(dx_layer >= 1)
+			if(layer >= 1)
 			{
 				const uint32_t idesc_x = instr_desc(kTile, kHidden);
-				const uint32_t w_base = smem_u32(smem + kOffBw + (dx_layer - 1) * kBwHidden);
+				const uint32_t w_base = smem_u32(smem + kOffBw + (layer - 1) * kBwHidden);
 				for(uint32_t ks = 0; ks < n_out / 16u; ++ks)
 				{
-					const uint64_t ad = smem_desc(a_g + ks * 2u * kLboG, kLboG, 128u);
-					const uint64_t bd = smem_desc(w_base + ks * 2u * kLboW, kLboW, 128u);
-					mma_bf16(tmem + kColAcc, ad, bd, idesc_x, ks > 0 ? 1u : 0u);
+					mma_bf16(tmem + kColAcc, smem_desc(a_g + ks * 2u * kLboG, kLboG, 128u),
+					         smem_desc(w_base + ks * 2u * kLboW, kLboW, 128u), idesc_x, ks > 0 ? 1u : 0u);
 				}
+				weight_chain(xt, col_w(layer), n_out, acc_w);
+			}
+			else
+			{
+				weight_chain(xt, kColW0a, kHidden, acc_w);
+				weight_chain(xt + kXtBytes, kColW0b, kHidden, acc_w);
 			}
 			mma_commit(bar);
 		}
@@ -466,28 +557,73 @@ backward_tc_kernel(const float* __restrict__ params, const float* __restrict__ f
 	bool first = true;
 	for(uint32_t tile = blockIdx.x; tile < num_tiles && !failed; tile += gridDim.x, first = false)
 	{
-		const uint32_t row = tile * kTile + tid;
+		const uint32_t row = tile * kTile + r;
 		const bool valid = row < n;
 
-		// ---- d loss / d raw outputs (48 columns, the last 8 zero)
-		float g[kHidden];
-		#pragma unroll
-		for(int c = 0; c < kHidden; ++c)
+		// this thread's columns of X_l (l = layer + 1: the activations of hidden layer `layer`)
+		auto load_x = [&](int layer, uint4* q)
 		{
-			g[c] = 0.0f;
-		}
-		float loss_term = 0.0f;
-		if(valid)
-		{
-			float raw[kOut];
+			const uint4* src = reinterpret_cast<const uint4*>(acts + (static_cast<size_t>(row) * kHiddenLayers + layer) * kHidden + c0);
 			#pragma unroll
-			for(int c = 0; c < kOut; ++c)
+			for(int c = 0; c < kCols / 8; ++c)
 			{
-				raw[c] = raw_out[static_cast<size_t>(row) * kOut + c];
+				q[c] = valid ? __ldg(src + c) : make_uint4(0u, 0u, 0u, 0u);
 			}
-			const float4 dw = dirw[row];
-			const float scale = -dw.w / fmaxf(*total_weight, 1e-30f);
-			output_gradient(raw, v3(dw.x, dw.y, dw.z), scale, g, &loss_term);
+		};
+		uint4 xq[kCols / 8];
+		load_x(3, xq);
+		float f7[kInputs];
+		#pragma unroll
+		for(int i = 0; i < kInputs; ++i)
+		{
+			f7[i] = valid ? __ldg(features + static_cast<size_t>(row) * 8 + i) : 0.0f;
+		}
+
+		// ---- d loss / d raw outputs: columns 20 part .. 20 part + 19 of 48 (the last 8 zero)
+		float loss_term = 0.0f;
+		{
+			float raw[20], g[20];
+			V3 d = v3(0.0f, 0.0f, 1.0f);
+			float scale = 0.0f;
+			#pragma unroll
+			for(int c = 0; c < 5; ++c)
+			{
+				const float4 q = valid ? __ldg(reinterpret_cast<const float4*>(raw_out + static_cast<size_t>(row) * kOut + 20u * part) + c)
+				                       : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+				raw[4 * c] = q.x; raw[4 * c + 1] = q.y; raw[4 * c + 2] = q.z; raw[4 * c + 3] = q.w;
+			}
+			if(valid)
+			{
+				const float4 dw = __ldg(dirw + row);
+				d = v3(dw.x, dw.y, dw.z);
+				scale = -dw.w / fmaxf(*total_weight, 1e-30f);
+			}
+			output_gradient_half(raw, d, scale, valid, part, xch + 3u * (part * kTile + r), xch + 3u * ((1u - part) * kTile + r),
+			                     g, &loss_term);
+			#pragma unroll
+			for(int o = 0; o < 20; ++o)
+			{
+				st_bf16(gt, core_offset_lbo(20u * part + static_cast<uint32_t>(o), r, kLboGT), g[o]);
+			}
+			if(part == 1u)
+			{
+				#pragma unroll
+				for(int o = kOut; o < kOutPad; ++o)
+				{
+					st_bf16(gt, core_offset_lbo(static_cast<uint32_t>(o), r, kLboGT), 0.0f);
+				}
+			}
+			// the sample's row of G, 4 columns at a time (20 is not a multiple of 8)
+			#pragma unroll
+			for(int c = 0; c < 5; ++c)
+			{
+				*reinterpret_cast<uint2*>(gbuf + core_offset_lbo(r, 20u * part + 4u * c, kLboG)) =
+					make_uint2(pack_bf16x2(g[4 * c], g[4 * c + 1]), pack_bf16x2(g[4 * c + 2], g[4 * c + 3]));
+			}
+			if(part == 1u)
+			{
+				*reinterpret_cast<uint4*>(gbuf + core_offset_lbo(r, kOut, kLboG)) = make_uint4(0u, 0u, 0u, 0u);
+			}
 		}
 		for(int o = 16; o > 0; o >>= 1)
 		{
@@ -498,154 +634,127 @@ backward_tc_kernel(const float* __restrict__ params, const float* __restrict__ f
 			atomicAdd(loss, loss_term);
 		}
 
-		// ---- layers 4..1: dW_l and dX_l together
-		for(int l = 4; l >= 1 && !failed; --l)
+		// ---- layers 4..1: dX_l and dW_l together
+		for(int l = 4; l >= 1; --l)
 		{
 			const uint32_t n_out = l == 4 ? static_cast<uint32_t>(kOutPad) : static_cast<uint32_t>(kHidden);
-			float x[kHidden];
-			const uint4* src = reinterpret_cast<const uint4*>(acts + (static_cast<size_t>(row) * kHiddenLayers + (l - 1)) * kHidden);
+			// X_l^T (+ the ones row); a BF16 activation is positive where its bits are neither 0 nor a sign
+			uint32_t positive = 0u;
 			#pragma unroll
-			for(int c = 0; c < kHidden / 8; ++c)
+			for(int c = 0; c < kCols / 8; ++c)
 			{
-				const uint4 q = valid ? src[c] : make_uint4(0u, 0u, 0u, 0u);
-				const uint32_t w4[4] = {q.x, q.y, q.z, q.w};
+				const uint32_t w4[4] = {xq[c].x, xq[c].y, xq[c].z, xq[c].w};
 				#pragma unroll
-				for(int j = 0; j < 4; ++j)
+				for(int j = 0; j < 8; ++j)
 				{
-					x[8 * c + 2 * j] = __bfloat162float(__ushort_as_bfloat16(static_cast<unsigned short>(w4[j] & 0xFFFFu)));
-					x[8 * c + 2 * j + 1] = __bfloat162float(__ushort_as_bfloat16(static_cast<unsigned short>(w4[j] >> 16)));
+					const uint16_t bits = static_cast<uint16_t>(w4[j / 2] >> (16 * (j & 1)));
+					const int f = 8 * c + j;
+					*reinterpret_cast<uint16_t*>(xt + core_offset_lbo(c0 + static_cast<uint32_t>(f), r, kLboXT)) = bits;
+					positive |= (bits != 0u && bits < 0x8000u) ? 1u << f : 0u;
 				}
 			}
-			// X_l^T (+ the ones row) and G_l^T, transposed; G_l as this sample's row
-			#pragma unroll
-			for(int f = 0; f < kHidden; ++f)
+			if(part == 0u)
 			{
-				st_bf16(xt, core_offset_lbo(static_cast<uint32_t>(f), tid, kLboXT), x[f]);
+				st_bf16(xt, core_offset_lbo(kHidden, r, kLboXT), 1.0f);
 			}
-			st_bf16(xt, core_offset_lbo(kHidden, tid, kLboXT), 1.0f);
-			#pragma unroll
-			for(int o = 0; o < kHidden; ++o)
+			if(l > 1)
 			{
-				if(o < static_cast<int>(n_out))
-				{
-					st_bf16(gt, core_offset_lbo(static_cast<uint32_t>(o), tid, kLboGT), g[o]);
-				}
+				load_x(l - 2, xq);   // the next round's, in flight while this one's MMAs run
 			}
-			#pragma unroll
-			for(int c = 0; c < kHidden / 8; ++c)
-			{
-				if(c * 8 < static_cast<int>(n_out))
-				{
-					uint4 q;
-					q.x = pack_bf16x2(g[8 * c + 0], g[8 * c + 1]);
-					q.y = pack_bf16x2(g[8 * c + 2], g[8 * c + 3]);
-					q.z = pack_bf16x2(g[8 * c + 4], g[8 * c + 5]);
-					q.w = pack_bf16x2(g[8 * c + 6], g[8 * c + 7]);
-					*reinterpret_cast<uint4*>(gbuf + core_offset_lbo(tid, static_cast<uint32_t>(8 * c), kLboG)) = q;
-				}
-			}
-			if(!run(col_w(l), n_out, !first, l))
+			if(!run(l, n_out, !first))
 			{
 				failed = true;
 				break;
 			}
-			// G_l-1 = dX_l through the ReLU that produced X_l
-			float acc[kHidden];
-			#pragma unroll
-			for(int c = 0; c < 4; ++c)
-			{
-				tmem_ld16(tmem_row + kColAcc + c * 16, acc + c * 16);
-			}
+			// G_l-1 = dX_l through the ReLU that produced X_l, staged for the next round
+			float g[kCols];
+			tmem_ld16(tmem_row + kColAcc + c0, g);
+			tmem_ld16(tmem_row + kColAcc + c0 + 16u, g + 16);
 			tmem_wait_ld();
 			#pragma unroll
-			for(int c = 0; c < kHidden; ++c)
+			for(int c = 0; c < kCols; ++c)
 			{
-				g[c] = x[c] > 0.0f ? acc[c] : 0.0f;
+				g[c] = (positive >> c) & 1u ? g[c] : 0.0f;
+				st_bf16(gt, core_offset_lbo(c0 + static_cast<uint32_t>(c), r, kLboGT), g[c]);
 			}
-			fence_before_sync();
-			__syncthreads();   // every thread's accumulator row is read before the next chain
+			#pragma unroll
+			for(int c = 0; c < kCols / 8; ++c)
+			{
+				*reinterpret_cast<uint4*>(gbuf + core_offset_lbo(r, c0 + 8u * c, kLboG)) = pack8(g + 8 * c);
+			}
 		}
 		if(failed)
 		{
 			break;
 		}
 
-		// ---- layer 0: dW_0 in two halves of its 224 one-blob inputs
-		float f7[kInputs];
+		// ---- layer 0: dW_0 of its 224 one-blob inputs, encoded as the forward pass encodes them; part 0
+		//      inputs 0, 2, 4 and 6, part 1 the others (unrolled so that f7 stays in registers)
 		#pragma unroll
 		for(int i = 0; i < kInputs; ++i)
 		{
-			f7[i] = valid ? features[static_cast<size_t>(row) * 8 + i] : 0.0f;
-		}
-		#pragma unroll
-		for(int o = 0; o < kHidden; ++o)
-		{
-			st_bf16(gt, core_offset_lbo(static_cast<uint32_t>(o), tid, kLboGT), g[o]);
-		}
-		// unrolled over the inputs so that f7 stays in registers (indexed at run time it went to
-		// local memory)
-		#pragma unroll
-		for(int half = 0; half < 2; ++half)
-		{
-			const int k0 = half * 128;
-			#pragma unroll
-			for(int i = half * 4; i < (half == 0 ? 4 : kInputs); ++i)
+			if((i & 1) == static_cast<int>(part))
 			{
-				#pragma unroll 8
-				for(int b = 0; b < kBins; ++b)
+				const float s32 = f7[i] * static_cast<float>(kBins) - 0.5f;
+				#pragma unroll
+				for(int c = 0; c < kBins / 8; ++c)
 				{
-					st_bf16(xt, core_offset_lbo(static_cast<uint32_t>(i * kBins + b - k0), tid, kLboXT), one_blob(f7[i], b));
+					const float z0 = s32 - static_cast<float>(c * 8);
+					float e = __expf(-0.5f * z0 * z0);
+					float ratio = __expf(z0 - 0.5f);
+					#pragma unroll
+					for(int j = 0; j < 8; ++j)
+					{
+						const uint32_t k = static_cast<uint32_t>(i * kBins + c * 8 + j);
+						st_bf16(k < 128u ? xt : xt + kXtBytes, core_offset_lbo(k & 127u, r, kLboXT), valid ? e : 0.0f);
+						e *= ratio;
+						ratio *= 0.36787944117144233f;   // e^-1
+					}
 				}
 			}
-			if(half == 1)
-			{
-				st_bf16(xt, core_offset_lbo(static_cast<uint32_t>(kIn - 128), tid, kLboXT), 1.0f);
-			}
-			if(!run(half == 0 ? kColW0a : kColW0b, kHidden, !first, 0))
-			{
-				failed = true;
-				break;
-			}
-			fence_before_sync();
-			__syncthreads();
+		}
+		if(part == 1u)
+		{
+			st_bf16(xt + kXtBytes, core_offset_lbo(static_cast<uint32_t>(kIn - 128), r, kLboXT), 1.0f);
+		}
+		if(!run(0, kHidden, !first))
+		{
+			failed = true;
+			break;
 		}
 	}
 
 	if(!failed)
 	{
-		// ---- the CTA's weight gradients to global memory: thread t holds row t of each block
-		auto flush = [&](uint32_t col, uint32_t n_out, int w_off, int b_off, uint32_t rows, uint32_t bias_row,
-		                 uint32_t first_input, uint32_t out_stride)
+		// ---- the CTA's weight gradients: thread t and t + 128 hold row t of each block, half of its
+		//      columns each
+		float* const out = partials + static_cast<size_t>(blockIdx.x) * kNumParams;
+		auto flush = [&](uint32_t col, int w_off, int b_off, uint32_t rows, uint32_t bias_row, uint32_t first_input,
+		                 uint32_t out_stride)
 		{
-			float v[kHidden];
-			for(uint32_t c = 0; c < n_out; c += 16)
-			{
-				tmem_ld16(tmem_row + col + c, v + c);
-			}
+			float v[kCols];
+			tmem_ld16(tmem_row + col + c0, v);
+			tmem_ld16(tmem_row + col + c0 + 16u, v + 16);
 			tmem_wait_ld();
-			if(tid < rows)
+			float* const dst = r < rows ? out + w_off + (first_input + r) * out_stride : out + b_off;
+			if(r < rows || r == bias_row)
 			{
-				float* dst = grads + w_off + (first_input + tid) * out_stride;
-				for(uint32_t c = 0; c < out_stride; ++c)
+				#pragma unroll
+				for(uint32_t c = 0; c < kCols; c += 8u)
 				{
-					if(v[c] != 0.0f) { atomicAdd(dst + c, v[c]); }
-				}
-			}
-			else if(tid == bias_row)
-			{
-				for(uint32_t c = 0; c < out_stride; ++c)
-				{
-					if(v[c] != 0.0f) { atomicAdd(grads + b_off + c, v[c]); }
+					if(c0 + c < out_stride)
+					{
+						st_global8(dst + c0 + c, v + c);
+					}
 				}
 			}
 		};
-		flush(kColW0a, kHidden, kOffW0, kOffB0, 128u, 0xFFFFFFFFu, 0u, kHidden);
-		flush(kColW0b, kHidden, kOffW0, kOffB0, static_cast<uint32_t>(kIn - 128), static_cast<uint32_t>(kIn - 128),
-		      128u, kHidden);
-		flush(col_w(1), kHidden, kOffW1, kOffB1, kHidden, kHidden, 0u, kHidden);
-		flush(col_w(2), kHidden, kOffW2, kOffB2, kHidden, kHidden, 0u, kHidden);
-		flush(col_w(3), kHidden, kOffW3, kOffB3, kHidden, kHidden, 0u, kHidden);
-		flush(col_w(4), kOutPad, kOffW4, kOffB4, kHidden, kHidden, 0u, kOut);
+		flush(kColW0a, kOffW0, kOffB0, 128u, 0xFFFFFFFFu, 0u, kHidden);
+		flush(kColW0b, kOffW0, kOffB0, static_cast<uint32_t>(kIn - 128), static_cast<uint32_t>(kIn - 128), 128u, kHidden);
+		flush(col_w(1), kOffW1, kOffB1, kHidden, kHidden, 0u, kHidden);
+		flush(col_w(2), kOffW2, kOffB2, kHidden, kHidden, 0u, kHidden);
+		flush(col_w(3), kOffW3, kOffB3, kHidden, kHidden, 0u, kHidden);
+		flush(col_w(4), kOffW4, kOffB4, kHidden, kHidden, 0u, kOut);
 	}
 	else if(tid == 0)
 	{
@@ -661,23 +770,68 @@ backward_tc_kernel(const float* __restrict__ params, const float* __restrict__ f
 
 }// end namespace tcb
 
-__global__ void adam_kernel(float* __restrict__ params, float* __restrict__ grads, float* __restrict__ m,
-                            float* __restrict__ v, uint32_t count, float lr, float beta1, float beta2,
-                            float eps, const uint32_t* __restrict__ step)
+// CTAs of the backward kernel that had a tile, each with a row of gradient sums in `partials`.
+__device__ __forceinline__ uint32_t partial_rows(uint32_t n_max, const uint32_t* d_n, uint32_t grid)
 {
+	const uint32_t n = d_n ? min(*d_n, n_max) : n_max;
+	return min((n + kTile - 1u) / kTile, grid);
+}
+
+// The gradient of parameter i: the CTAs' sums, in their order (eight loads in flight).
+__device__ __forceinline__ float sum_partials(const float* __restrict__ partials, uint32_t rows, uint32_t i)
+{
+	float s = 0.0f;
+	uint32_t b = 0;
+	for(; b + 8u <= rows; b += 8u)
+	{
+		float v[8];
+		#pragma unroll
+		for(uint32_t k = 0; k < 8u; ++k)
+		{
+			v[k] = __ldg(partials + static_cast<size_t>(b + k) * kNumParams + i);
+		}
+		s += ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+	}
+	for(; b < rows; ++b)
+	{
+		s += __ldg(partials + static_cast<size_t>(b) * kNumParams + i);
+	}
+	return s;
+}
+
+__global__ void reduce_partials_kernel(const float* __restrict__ partials, uint32_t n_max, const uint32_t* __restrict__ d_n,
+                                       uint32_t grid, float* __restrict__ grads)
+{
+	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+	if(i < kNumParams)
+	{
+		grads[i] += sum_partials(partials, partial_rows(n_max, d_n, grid), i);
+	}
+}
+
+// Adds up the step's gradient, applies Adam and writes the new weight to the packed image the network
+// kernels read, in one launch.
+__global__ void adam_kernel(float* __restrict__ params, const float* __restrict__ partials, uint32_t n_max,
+                            const uint32_t* __restrict__ d_n, uint32_t grid, float* __restrict__ m,
+                            float* __restrict__ v, float lr, float beta1, float beta2, float eps,
+                            const uint32_t* __restrict__ step, unsigned char* __restrict__ image)
+{
+	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+	if(i >= kNumParams)
+	{
+		return;
+	}
 	const float t = static_cast<float>(*step + 1u);
 	const float bias1 = 1.0f - powf(beta1, t);
 	const float bias2 = 1.0f - powf(beta2, t);
-	for(uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
-	{
-		const float g = grads[i];
-		const float mi = beta1 * m[i] + (1.0f - beta1) * g;
-		const float vi = beta2 * v[i] + (1.0f - beta2) * g * g;
-		m[i] = mi;
-		v[i] = vi;
-		params[i] -= lr * (mi / bias1) / (sqrtf(vi / bias2) + eps);
-		grads[i] = 0.0f;
-	}
+	const float g = sum_partials(partials, partial_rows(n_max, d_n, grid), i);
+	const float mi = beta1 * m[i] + (1.0f - beta1) * g;
+	const float vi = beta2 * v[i] + (1.0f - beta2) * g * g;
+	m[i] = mi;
+	v[i] = vi;
+	const float w = params[i] - lr * (mi / bias1) / (sqrtf(vi / bias2) + eps);
+	params[i] = w;
+	store_image(image, i, w);
 }
 
 __global__ void step_kernel(uint32_t* step)
@@ -685,10 +839,22 @@ __global__ void step_kernel(uint32_t* step)
 	++*step;
 }
 
+uint32_t backward_grid(uint32_t n)
+{
+	// one CTA per SM: a batch of up to one tile per SM runs in one round of tiles; larger batches keep
+	// their weight gradients in TMEM across each CTA's tiles
+	return std::max(1u, std::min((n + kTile - 1u) / kTile, static_cast<uint32_t>(sm_count())));
+}
+
 }// end anonymous namespace
 
+std::size_t partial_floats(uint32_t n)
+{
+	return static_cast<std::size_t>(backward_grid(n)) * kNumParams;
+}
+
 void launch_gradients(const float* d_params, const unsigned char* d_image, const float* d_features,
-                      const float4* d_dirw, uint32_t n, float* d_raw, __nv_bfloat16* d_acts,
+                      const float4* d_dirw, uint32_t n, float* d_raw, __nv_bfloat16* d_acts, float* d_partials,
                       float* d_grads, float* d_loss, float* d_total, uint32_t* d_error, cudaStream_t s,
                       const uint32_t* d_n, float clamp_factor, bool tensor_cores)
 {
@@ -717,14 +883,15 @@ void launch_gradients(const float* d_params, const unsigned char* d_image, const
 			return true;
 		}();
 		(void)configured_tc;
-		// one CTA per SM: a batch of up to one tile per SM runs in one round of tiles; larger
-		// batches keep their weight gradients in TMEM across each CTA's tiles, and every CTA adds
-		// them to global memory once
-		const uint32_t tiles = (n + kTile - 1) / kTile;
-		const uint32_t grid = std::max(1u, std::min(tiles, static_cast<uint32_t>(sm_count())));
+		const uint32_t grid = backward_grid(n);
 		tcb::backward_tc_kernel<<<grid, tcb::kThreads, tcb::kSmemBytes, s>>>(d_params, d_features, d_dirw, d_raw, d_acts,
-		                                                                     n, d_n, d_total, d_grads, d_loss, d_error);
+		                                                                     n, d_n, d_total, d_partials, d_loss, d_error);
 		PG_CUDA_CHECK(cudaGetLastError());
+		if(d_grads)
+		{
+			reduce_partials_kernel<<<(kNumParams + 127) / 128, 128, 0, s>>>(d_partials, n, d_n, grid, d_grads);
+			PG_CUDA_CHECK(cudaGetLastError());
+		}
 		return;
 	}
 	constexpr int smem_bytes = 2 * kBlock * kPitch * sizeof(float);
@@ -739,9 +906,11 @@ void launch_gradients(const float* d_params, const unsigned char* d_image, const
 	PG_CUDA_CHECK(cudaGetLastError());
 }
 
-void launch_adam(float* d_params, float* d_grads, float* d_m, float* d_v, uint32_t* d_step, float lr, cudaStream_t s)
+void launch_adam(float* d_params, const float* d_partials, uint32_t n, const uint32_t* d_n, float* d_m, float* d_v,
+                 uint32_t* d_step, unsigned char* d_image, float lr, cudaStream_t s)
 {
-	adam_kernel<<<64, 256, 0, s>>>(d_params, d_grads, d_m, d_v, kNumParams, lr, 0.9f, 0.999f, 1e-8f, d_step);
+	adam_kernel<<<(kNumParams + 127) / 128, 128, 0, s>>>(d_params, d_partials, n, d_n, backward_grid(n), d_m, d_v, lr, 0.9f,
+	                                                     0.999f, 1e-8f, d_step, d_image);
 	PG_CUDA_CHECK(cudaGetLastError());
 	step_kernel<<<1, 1, 0, s>>>(d_step);
 	PG_CUDA_CHECK(cudaGetLastError());
@@ -779,6 +948,7 @@ int pgpu_guide_gradients_ex(const float* params, const float* features, const fl
 		ScratchBuffer<unsigned char> d_image(guide::image_bytes());
 		ScratchBuffer<float> d_feat(n * 8), d_raw(n * guide::kOut), d_scalars(2);
 		ScratchBuffer<float4> d_dirw(n);
+		ScratchBuffer<float> d_partials(guide::partial_floats(static_cast<uint32_t>(n)));
 		ScratchBuffer<__nv_bfloat16> d_acts(n * guide::kHiddenLayers * guide::kHidden);
 		ScratchBuffer<uint32_t> d_err(1);
 		PG_CUDA_CHECK(cudaMemsetAsync(d_err.get(), 0, sizeof(uint32_t), s));
@@ -788,7 +958,7 @@ int pgpu_guide_gradients_ex(const float* params, const float* features, const fl
 		guide::upload_rows(features, dirs, weights, n, d_feat.get(), d_dirw.get(), s);
 		guide::pack_image(d_params.get(), d_image.get(), s);
 		guide::launch_gradients(d_params.get(), d_image.get(), d_feat.get(), d_dirw.get(), static_cast<uint32_t>(n),
-		                        d_raw.get(), d_acts.get(), d_grads.get(), d_scalars.get(), d_scalars.get() + 1,
+		                        d_raw.get(), d_acts.get(), d_partials.get(), d_grads.get(), d_scalars.get(), d_scalars.get() + 1,
 		                        d_err.get(), s, nullptr, 0.0f, (flags & PG_GUIDE_BACKWARD_CUDA_CORES) == 0u);
 		float scalars[2] = {0.0f, 0.0f};
 		uint32_t err = 0;
@@ -820,7 +990,7 @@ int pgpu_guide_train(float* params, const float* features, const float* dirs, co
 		require_device();
 		cudaStream_t s = library_stream();
 		const uint32_t b = static_cast<uint32_t>(std::min<uint64_t>(batch, n));
-		ScratchBuffer<float> d_params(guide::kNumParams), d_grads(guide::kNumParams), d_m(guide::kNumParams),
+		ScratchBuffer<float> d_params(guide::kNumParams), d_partials(guide::partial_floats(b)), d_m(guide::kNumParams),
 			d_v(guide::kNumParams);
 		ScratchBuffer<unsigned char> d_image(guide::image_bytes());
 		ScratchBuffer<float> d_feat(n * 8), d_raw(static_cast<std::size_t>(b) * guide::kOut), d_scalars(2 * static_cast<std::size_t>(steps));
@@ -829,21 +999,21 @@ int pgpu_guide_train(float* params, const float* features, const float* dirs, co
 		ScratchBuffer<uint32_t> d_err(1), d_step(1);
 		PG_CUDA_CHECK(cudaMemsetAsync(d_err.get(), 0, sizeof(uint32_t), s));
 		PG_CUDA_CHECK(cudaMemsetAsync(d_step.get(), 0, sizeof(uint32_t), s));
-		PG_CUDA_CHECK(cudaMemsetAsync(d_grads.get(), 0, d_grads.bytes(), s));
 		PG_CUDA_CHECK(cudaMemsetAsync(d_m.get(), 0, d_m.bytes(), s));
 		PG_CUDA_CHECK(cudaMemsetAsync(d_v.get(), 0, d_v.bytes(), s));
 		PG_CUDA_CHECK(cudaMemsetAsync(d_scalars.get(), 0, d_scalars.bytes(), s));
 		PG_CUDA_CHECK(cudaMemcpyAsync(d_params.get(), params, d_params.bytes(), cudaMemcpyHostToDevice, s));
 		guide::upload_rows(features, dirs, weights, n, d_feat.get(), d_dirw.get(), s);
+		guide::pack_image(d_params.get(), d_image.get(), s);
 		for(uint32_t step = 0; step < steps; ++step)
 		{
 			const uint32_t first = static_cast<uint32_t>((static_cast<uint64_t>(step) * b) % n);
 			const uint32_t count = std::min<uint32_t>(b, static_cast<uint32_t>(n - first));
-			guide::pack_image(d_params.get(), d_image.get(), s);
 			guide::launch_gradients(d_params.get(), d_image.get(), d_feat.get() + static_cast<size_t>(first) * 8,
-			                        d_dirw.get() + first, count, d_raw.get(), d_acts.get(), d_grads.get(),
+			                        d_dirw.get() + first, count, d_raw.get(), d_acts.get(), d_partials.get(), nullptr,
 			                        d_scalars.get() + 2 * step, d_scalars.get() + 2 * step + 1, d_err.get(), s);
-			guide::launch_adam(d_params.get(), d_grads.get(), d_m.get(), d_v.get(), d_step.get(), lr, s);
+			guide::launch_adam(d_params.get(), d_partials.get(), count, nullptr, d_m.get(), d_v.get(), d_step.get(),
+			                   d_image.get(), lr, s);
 		}
 		std::vector<float> scalars(2 * static_cast<std::size_t>(steps));
 		uint32_t err = 0;

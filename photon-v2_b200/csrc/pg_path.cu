@@ -1784,6 +1784,7 @@ void RenderScene::ensure_guiding(uint32_t capacity)
 		m_traw.resize(static_cast<std::size_t>(batch) * guide::kOut);
 		m_tdirw.resize(batch);
 		m_tacts.resize(static_cast<std::size_t>(batch) * guide::kHiddenLayers * guide::kHidden);
+		m_gpartials.resize(guide::partial_floats(batch));
 	}
 	if(!m_guide_ready)
 	{
@@ -1817,7 +1818,6 @@ void RenderScene::ensure_guiding(uint32_t capacity)
 		m_gparams.resize(guide::kNumParams);
 		m_gm.resize(guide::kNumParams);
 		m_gv.resize(guide::kNumParams);
-		m_ggrads.resize(guide::kNumParams);
 		m_gscalars.resize(4);   // step loss, weight total, loss sum over the render, steps with samples
 		m_gimage.resize(guide::image_bytes());
 		m_gstep.resize(1);
@@ -1825,7 +1825,6 @@ void RenderScene::ensure_guiding(uint32_t capacity)
 		PG_CUDA_CHECK(cudaMemcpyAsync(m_gparams.get(), p.data(), m_gparams.bytes(), cudaMemcpyHostToDevice, st));
 		PG_CUDA_CHECK(cudaMemsetAsync(m_gm.get(), 0, m_gm.bytes(), st));
 		PG_CUDA_CHECK(cudaMemsetAsync(m_gv.get(), 0, m_gv.bytes(), st));
-		PG_CUDA_CHECK(cudaMemsetAsync(m_ggrads.get(), 0, m_ggrads.bytes(), st));
 		PG_CUDA_CHECK(cudaMemsetAsync(m_gscalars.get(), 0, m_gscalars.bytes(), st));
 		PG_CUDA_CHECK(cudaMemsetAsync(m_gstep.get(), 0, m_gstep.bytes(), st));
 		PG_CUDA_CHECK(cudaMemsetAsync(m_gerr.get(), 0, m_gerr.bytes(), st));
@@ -2703,12 +2702,11 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 			// next period
 			PG_CUDA_CHECK(cudaMemsetAsync(m_gscalars.get(), 0, sizeof(float), st));
 			guide::launch_gradients(m_gparams.get(), m_gimage.get(), m_tfeat.get(), m_tdirw.get(), train_cap,
-			                        m_traw.get(), reinterpret_cast<__nv_bfloat16*>(m_tacts.get()), m_ggrads.get(),
+			                        m_traw.get(), reinterpret_cast<__nv_bfloat16*>(m_tacts.get()), m_gpartials.get(), nullptr,
 			                        m_gscalars.get(), m_gscalars.get() + 1, m_gerr.get(), st, &d_counters->n_train,
 			                        m_guide_params.clamp);
-			guide::launch_adam(m_gparams.get(), m_ggrads.get(), m_gm.get(), m_gv.get(), m_gstep.get(),
-			                   m_guide_params.lr, st);
-			guide::pack_image(m_gparams.get(), m_gimage.get(), st);
+			guide::launch_adam(m_gparams.get(), m_gpartials.get(), train_cap, &d_counters->n_train, m_gm.get(), m_gv.get(),
+			                   m_gstep.get(), m_gimage.get(), m_guide_params.lr, st);
 			guide_loss_kernel<<<1, 1, 0, st>>>(m_gscalars.get(), &d_counters->n_train);
 			PG_CUDA_CHECK(cudaGetLastError());
 		}
@@ -2889,7 +2887,7 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 	{
 		// begin, trace + classify, shade per material kind (+ refine in the iterative
 		// mode); guide query + forward; training: weight sums (and clamp), forward, backward, Adam,
-		// step, repack, loss
+		// step, loss
 		const unsigned long long per_iteration = 3ull + (classify ? 1ull : 0ull) + ((kinds >> kShadeConductor) & 1u) + ((kinds >> kShadeDielectric) & 1u) +
 		                                         (params.refine_mode == PG_REFINE_ITERATIVE ? 1ull : 0ull) +
 		                                         (guided ? 2ull : 0ull);

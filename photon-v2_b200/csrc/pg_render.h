@@ -487,7 +487,7 @@ private:
 	DeviceBuffer<float>    m_tfeat, m_traw;
 	DeviceBuffer<float4>   m_tdirw;
 	DeviceBuffer<uint16_t> m_tacts;
-	DeviceBuffer<float>    m_gparams, m_gm, m_gv, m_ggrads, m_gscalars;
+	DeviceBuffer<float>    m_gparams, m_gm, m_gv, m_gpartials, m_gscalars;
 	DeviceBuffer<unsigned char> m_gimage;
 	DeviceBuffer<uint32_t> m_gstep, m_gerr;
 	float m_last_guide_loss = 0.0f;
