@@ -601,10 +601,7 @@ begin_kernel(const RenderCounters* __restrict__ prev, RenderCounters* __restrict
 		const V3 d = -recv;
 
 		cur.path[i] = p;
-		cur.meta[i] = sid << kMetaSceneShift;
-		cur.thr[i] = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
-		cur.rad[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-		cur.prev[i] = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
+		cur.meta[i] = kMetaCamera | (sid << kMetaSceneShift);   // (its thr, rad and prev go without saying)
 		cur.ray_o[i] = make_float4(cam.pos[0], cam.pos[1], cam.pos[2], 0.0f);
 		cur.ray_d[i] = make_float4(d.x, d.y, d.z, kFloatMax);
 	}
@@ -826,9 +823,16 @@ shade_kernel(ShadeArgs a)
 		const FilmView& film = MULTI ? a.batch.scenes[sid].film : a.film;
 		const uint32_t width_height = MULTI ? a.batch.scenes[sid].width_height : a.width_height;
 		const uint64_t first_global = MULTI ? a.batch.scenes[sid].first_global : consts.first_global;
-		const float4 thr4 = ld4(a.cur.thr + i);
-		const float4 rad4 = ld4(a.cur.rad + i);
-		const float4 prev4 = ld4(a.cur.prev + i);
+		// a path that comes from the camera: throughput and continuation factor 1, no radiance yet
+		float4 thr4 = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+		float4 rad4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+		float4 prev4 = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
+		if(!(meta & kMetaCamera))
+		{
+			thr4 = ld4(a.cur.thr + i);
+			rad4 = ld4(a.cur.rad + i);
+			prev4 = ld4(a.cur.prev + i);
+		}
 		const float4 ro = ld4(a.cur.ray_o + i);
 		const float4 rd = ld4(a.cur.ray_d + i);
 		const uint2 hit = a.hits[i];

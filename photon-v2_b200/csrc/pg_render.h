@@ -342,6 +342,7 @@ constexpr uint32_t kMetaPrevNee = 1u << 8;      // the previous vertex used NEE 
 constexpr uint32_t kMetaStopAfter = 1u << 9;    // Russian roulette ended the path after this hit
 constexpr uint32_t kMetaGuideRec = 1u << 10;    // gf0/gf1 hold a guided vertex awaiting its training sample
 constexpr uint32_t kMetaGuideOpen = 1u << 11;   // gf0 holds an open training record (row, weight scale)
+constexpr uint32_t kMetaCamera = 1u << 12;      // a camera ray: the path's thr, rad and prev are not written
 constexpr uint32_t kTargetFinal = 0x80000000u;
 
 // Launcher implemented in pg_trace.cu (FMA-enabled traversal kernels); min_idle is the
