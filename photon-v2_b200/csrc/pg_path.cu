@@ -376,24 +376,36 @@ __global__ void count_inflight_kernel(const uint32_t* __restrict__ path, const R
 	}
 }
 
+// The paths generated so far: [first, end) of each wavefront (an empty range where there is none).
+struct PathRanges
+{
+	unsigned long long first[2];
+	unsigned long long end[2];
+};
+
 // The film's estimate over finished samples (HdrRgbFilm::developRegion, HdrRgbFilm.cpp:167-205,
 // on what the finished paths have deposited). The box film's W was raised by this render's spp
-// up front, so the samples of the render that have not finished -- not generated yet (path
-// indices from `generated` on; pixel = index mod wh) or still in flight -- come off it; the
-// 4 x 4 films only hold whole passes, whose W is exact.
+// up front, so the samples of the render that have not finished -- not generated yet (pixel = path
+// index mod wh) or still in flight -- come off it; the 4 x 4 films only hold whole passes, whose W
+// is exact.
 __global__ void develop_preview_kernel(const double* __restrict__ sums, const uint32_t* __restrict__ inflight,
-                                       uint32_t wh, uint32_t spp, unsigned long long generated, int box,
+                                       uint32_t wh, uint32_t spp, PathRanges generated, int box,
                                        float* __restrict__ rgb)
 {
-	const unsigned long long full = generated / wh;
-	const uint32_t part = static_cast<uint32_t>(generated % wh);
 	for(uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < wh; i += gridDim.x * blockDim.x)
 	{
 		const double4 s = reinterpret_cast<const double4*>(sums)[i];
 		double w = s.w;
 		if(box)
 		{
-			const unsigned long long gen = full + (i < part ? 1ull : 0ull);
+			unsigned long long gen = 0;
+			#pragma unroll
+			for(int v = 0; v < 2; ++v)
+			{
+				// indices below x that fall on pixel i: x / wh, and one more if i < x mod wh
+				gen += generated.end[v] / wh + (i < generated.end[v] % wh ? 1ull : 0ull);
+				gen -= generated.first[v] / wh + (i < generated.first[v] % wh ? 1ull : 0ull);
+			}
 			w -= static_cast<double>(spp) - static_cast<double>(gen) + static_cast<double>(inflight[i]);
 		}
 		const double rcp = w > 0.0 ? 1.0 / w : 0.0;
@@ -1667,7 +1679,7 @@ RenderScene::RenderScene(const SceneDesc& desc, float max_origin_abs)
 		for(int k = 0; k < 3; ++k) { m_dev.env_map.center[k] = desc.env_center[k]; }
 		m_dev.env_map.radius = static_cast<float>(std::sqrt(desc.env_area / (4.0 * 3.14159265358979323846)));
 	}
-	m_state.resize(1);
+	m_waves[0].stream = m_stream;
 	PG_CUDA_CHECK(cudaStreamSynchronize(st));
 
 	m_dev.nodes = m_geometry->nodes.get();
@@ -1683,18 +1695,21 @@ RenderScene::RenderScene(const SceneDesc& desc, float max_origin_abs)
 
 RenderScene::~RenderScene()
 {
-	if(m_exec)
+	for(Wave& w : m_waves)
 	{
-		cudaGraphExecDestroy(m_exec);
-	}
-	if(m_stream)
-	{
-		cudaStreamSynchronize(m_stream);
-		cudaStreamDestroy(m_stream);
-	}
-	if(m_host_state)
-	{
-		cudaFreeHost(m_host_state);
+		if(w.exec)
+		{
+			cudaGraphExecDestroy(w.exec);
+		}
+		if(w.stream)
+		{
+			cudaStreamSynchronize(w.stream);
+			cudaStreamDestroy(w.stream);
+		}
+		if(w.host_state)
+		{
+			cudaFreeHost(w.host_state);
+		}
 	}
 	for(cudaEvent_t e : m_events)
 	{
@@ -1705,14 +1720,13 @@ RenderScene::~RenderScene()
 	}
 }
 
-void RenderScene::ensure_capacity(uint32_t capacity, uint32_t grid)
+void RenderScene::ensure_capacity(uint32_t waves, uint32_t capacity, uint32_t grid)
 {
-	if(capacity <= m_capacity && grid == m_order_grid)
+	if(waves <= m_pool_waves && capacity <= m_capacity && grid == m_order_grid)
 	{
 		return;
 	}
 	++m_buffer_generation;
-	capacity = std::max(capacity, m_capacity);
 	// the slots the blocks of one residue visit in classify_kernel's grid-stride loop
 	const uint32_t rounds = (capacity + grid * kShadeBlock - 1u) / (grid * kShadeBlock);
 	m_order_list = (grid + kClassLists - 1u) / kClassLists * rounds * kShadeBlock;
@@ -1732,32 +1746,42 @@ void RenderScene::ensure_capacity(uint32_t capacity, uint32_t grid)
 			}
 			at += (n * sizeof(T) + 255u) / 256u * 256u;
 		};
-		for(int b = 0; b < 2; ++b)
+		for(uint32_t k = 0; k < waves; ++k)
 		{
-			carve(m_path[b], capacity);
-			carve(m_meta[b], capacity);
-			carve(m_thr[b], capacity);
-			carve(m_rad[b], capacity);
-			carve(m_prev[b], capacity);
-			carve(m_ro[b], capacity);
-			carve(m_rd[b], capacity);
-			carve(m_so[b], capacity);
-			carve(m_sd[b], capacity);
-			carve(m_sc[b], capacity);
-			carve(m_sr[b], capacity);
+			Wave& w = m_waves[k];
+			for(int b = 0; b < 2; ++b)
+			{
+				carve(w.path[b], capacity);
+				carve(w.meta[b], capacity);
+				carve(w.thr[b], capacity);
+				carve(w.rad[b], capacity);
+				carve(w.prev[b], capacity);
+				carve(w.ro[b], capacity);
+				carve(w.rd[b], capacity);
+				carve(w.so[b], capacity);
+				carve(w.sd[b], capacity);
+				carve(w.sc[b], capacity);
+				carve(w.sr[b], capacity);
+				carve(w.sid[b], capacity);
+			}
+			carve(w.hits, capacity);
+			carve(w.req_single, capacity);
+			carve(w.req_mutual, capacity);
+			carve(w.order, static_cast<std::size_t>(kOrderLists) * m_order_list);
 		}
-		carve(m_hits, capacity);
-		carve(m_req_single, capacity);
-		carve(m_req_mutual, capacity);
-		carve(m_order, static_cast<std::size_t>(kOrderLists) * m_order_list);
 		if(round == 0)
 		{
 			total = at;
-			m_capacity = 0;      // the old pool goes first
-			m_pool.release();
-			m_pool.resize(total);
+			if(total > m_pool.size())
+			{
+				m_capacity = 0;      // the old pool goes first
+				m_pool_waves = 0;
+				m_pool.release();
+				m_pool.resize(total);
+			}
 		}
 	}
+	m_pool_waves = waves;
 	m_capacity = capacity;
 	m_order_grid = grid;
 }
@@ -2384,14 +2408,14 @@ uint64_t float_bits(float v)
 
 }// end anonymous namespace
 
-// Captures `launches` (on the scene's stream; given the loop's handle) as the body of a loop on the
-// device and instantiates it as m_exec.
-void RenderScene::build_loop_graph(const std::function<void(cudaGraphConditionalHandle)>& launches)
+// Captures `launches` (on the wave's stream; given the loop's handle) as the body of a loop on the
+// device and instantiates it as the wave's graph.
+void RenderScene::build_loop_graph(Wave& wave, const std::function<void(cudaGraphConditionalHandle)>& launches)
 {
-	if(m_exec)
+	if(wave.exec)
 	{
-		PG_CUDA_CHECK(cudaGraphExecDestroy(m_exec));
-		m_exec = nullptr;
+		PG_CUDA_CHECK(cudaGraphExecDestroy(wave.exec));
+		wave.exec = nullptr;
 	}
 	struct GraphHolder
 	{
@@ -2408,7 +2432,7 @@ void RenderScene::build_loop_graph(const std::function<void(cudaGraphConditional
 	node.conditional.size = 1;
 	cudaGraphNode_t added;
 	PG_CUDA_CHECK(cudaGraphAddNode(&added, holder.g, nullptr, 0, &node));
-	PG_CUDA_CHECK(cudaStreamBeginCaptureToGraph(m_stream, node.conditional.phGraph_out[0], nullptr, nullptr, 0,
+	PG_CUDA_CHECK(cudaStreamBeginCaptureToGraph(wave.stream, node.conditional.phGraph_out[0], nullptr, nullptr, 0,
 	                                            cudaStreamCaptureModeThreadLocal));
 	try
 	{
@@ -2417,13 +2441,13 @@ void RenderScene::build_loop_graph(const std::function<void(cudaGraphConditional
 	catch(...)
 	{
 		cudaGraph_t body;
-		cudaStreamEndCapture(m_stream, &body);
+		cudaStreamEndCapture(wave.stream, &body);
 		(void)cudaGetLastError();
 		throw;
 	}
 	cudaGraph_t body;
-	PG_CUDA_CHECK(cudaStreamEndCapture(m_stream, &body));
-	PG_CUDA_CHECK(cudaGraphInstantiate(&m_exec, holder.g, 0));
+	PG_CUDA_CHECK(cudaStreamEndCapture(wave.stream, &body));
+	PG_CUDA_CHECK(cudaGraphInstantiate(&wave.exec, holder.g, 0));
 }
 
 float RenderScene::render_pass(const RenderParams& params, double* film_sums, const std::vector<BatchScene>* batch)
@@ -2458,34 +2482,67 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 	                                                                                             : lc.capacity, total));
 	const int sms = sm_count();
 	const int grid = sms * static_cast<int>(lc.blocks_per_sm);   // grid-stride kernels: 128-thread blocks
-	ensure_capacity(std::max<uint32_t>(capacity, 1024u), static_cast<uint32_t>(grid));
 	const int refill = static_cast<int>(lc.refill);
+	const bool guided = m_guide_params.enabled && params.estimator == PG_EST_BNEEPT;   // (BNEEPT only)
 
-	cudaStream_t st = m_stream;
-	PathBuffers buf[2];
-	for(int b = 0; b < 2; ++b)
+	// Two wavefronts, each with half of the paths and of the pool, run side by side on streams of their
+	// own: a traversal launch ends with a tail of its longest rays (a fifth of its time on the bench
+	// scene), in which the other wavefront's kernels take over the SMs that have run dry. That pays
+	// where the paths fill the pool at least twice (Cornell box at 64 samples 4.82 to 4.45 ms, bench scene
+	// at 16 samples 18.4 to 18.0 ms, 8 scenes in one wavefront 104.6 to 101.9 ms); below, the queues only
+	// drain, a half-empty launch takes as long as a full one, and one wavefront is better (slit room at
+	// 2 samples, which fill the pool once, 14.55 against 14.84 ms). Guided renders share a training
+	// batch and profiled ones time kernel by kernel: one wavefront.
+	const uint32_t waves = params.mode == PG_RENDER_GRAPH && !guided && total >= 2ull * capacity ? 2u : 1u;
+	const uint32_t wave_capacity = (capacity + waves - 1u) / waves;
+	ensure_capacity(waves, std::max<uint32_t>(wave_capacity, 1024u), static_cast<uint32_t>(grid));
+
+	cudaStream_t const st = m_stream;
+	// each wave's buffers by iteration parity, counter sets and pinned counters
+	struct WaveView
 	{
-		buf[b] = PathBuffers{m_path[b].get(), m_meta[b].get(), m_thr[b].get(), m_rad[b].get(),
-		                     m_prev[b].get(), m_ro[b].get(), m_rd[b].get()};
-	}
-	ShadowQueue sqs[2];
-	for(int b = 0; b < 2; ++b)
+		Wave*           wave;
+		PathBuffers     buf[2];
+		ShadowQueue     sqs[2];
+		RenderCounters* counters[2];
+		const RenderConsts* consts;
+		RenderCounters* host;
+		unsigned long long first, end;   // its paths
+		bool            done;
+	};
+	WaveView views[kMaxWaves];
+	for(uint32_t v = 0; v < waves; ++v)
 	{
-		sqs[b] = ShadowQueue{m_so[b].get(), m_sd[b].get(), m_sc[b].get()};
-		sqs[b].r = m_sr[b].get();
+		Wave& w = m_waves[v];
+		if(!w.stream)
+		{
+			PG_CUDA_CHECK(cudaStreamCreateWithFlags(&w.stream, cudaStreamNonBlocking));
+		}
+		w.state.resize(1);
+		if(!w.host_state)
+		{
+			PG_CUDA_CHECK(cudaMallocHost(&w.host_state, sizeof(RenderState)));
+		}
+		WaveView& x = views[v];
+		x = WaveView{};
+		x.wave = &w;
+		for(int b = 0; b < 2; ++b)
+		{
+			x.buf[b] = PathBuffers{w.path[b].get(), w.meta[b].get(), w.thr[b].get(), w.rad[b].get(),
+			                       w.prev[b].get(), w.ro[b].get(), w.rd[b].get()};
+			x.sqs[b] = ShadowQueue{w.so[b].get(), w.sd[b].get(), w.sc[b].get()};
+			x.sqs[b].r = w.sr[b].get();
+			x.sqs[b].sid = multi ? w.sid[b].get() : nullptr;
+			x.counters[b] = &w.state.get()->counters[1 - b];   // the iteration before the first: set 0
+		}
+		x.consts = &w.state.get()->consts;
+		x.host = &w.host_state->counters[0];
+		x.first = total * v / waves;
+		x.end = total * (v + 1u) / waves;
 	}
 	BatchView bview;
 	if(multi)
 	{
-		for(int b = 0; b < 2; ++b)
-		{
-			if(m_ssid[b].size() < m_capacity)
-			{
-				++m_buffer_generation;
-				m_ssid[b].resize(m_capacity);
-			}
-			sqs[b].sid = m_ssid[b].get();
-		}
 		if(m_batch_table.size() < batch->size())
 		{
 			++m_buffer_generation;
@@ -2506,27 +2563,23 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 	}
 	const uint64_t first_global = params.first_sample * wh;
 	// what changes from render to render goes through device memory, so that a scene's graph serves
-	// all its renders of one shape; the counters of the iteration before the first are set 0
-	if(!m_host_state)
+	// all its renders of one shape
+	for(uint32_t v = 0; v < waves; ++v)
 	{
-		PG_CUDA_CHECK(cudaMallocHost(&m_host_state, sizeof(RenderState)));
+		WaveView& x = views[v];
+		*x.host = RenderCounters{};
+		x.host->next_path = x.first;
+		x.host->total_paths = x.end;
+		x.host->pause_at = params.progress ? kFirstPause : 0xFFFFFFFFu;
+		x.host->pause_step = kFirstPause;
+		x.wave->host_state->consts = RenderConsts{params.seed, first_global};
+		PG_CUDA_CHECK(cudaMemcpyAsync(x.wave->state.get(), x.wave->host_state, kStateHead, cudaMemcpyHostToDevice, st));
 	}
-	RenderCounters* const host_counters = &m_host_state->counters[0];
-	*host_counters = RenderCounters{};
-	host_counters->total_paths = total;
-	host_counters->pause_at = params.progress ? kFirstPause : 0xFFFFFFFFu;
-	host_counters->pause_step = kFirstPause;
-	m_host_state->consts = RenderConsts{params.seed, first_global};
-	PG_CUDA_CHECK(cudaMemcpyAsync(m_state.get(), m_host_state, kStateHead, cudaMemcpyHostToDevice, st));
-	RenderCounters* const counters_of[2] = {&m_state.get()->counters[1], &m_state.get()->counters[0]};   // by parity
-	const RenderConsts* const consts = &m_state.get()->consts;
 	const bool counting = params.mode == PG_RENDER_COUNT;
 	// BVPTDL follows one BSDF-sampled bounce whatever the configured depth (BVPTDLEstimator.cpp:62-95)
 	const uint32_t max_bounces = params.estimator == PG_EST_BVPTDL ? 1u : params.max_bounces;
 
-	// learned guiding (BNEEPT only)
-	const bool guided = m_guide_params.enabled && params.estimator == PG_EST_BNEEPT;
-	// the vertices a guided render guides: those below this bounce (0: none)
+	// learned guiding: the vertices a guided render guides: those below this bounce (0: none)
 	const uint32_t guide_depth = !guided ? 0u
 	                             : (m_guide_params.depth == 0u || m_guide_params.depth > max_bounces ? max_bounces
 	                                                                                                : m_guide_params.depth);
@@ -2539,14 +2592,14 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 		train_cap = training ? std::max<uint32_t>(m_guide_params.batch, guide::kTile) : 0u;
 		for(int b = 0; b < 2; ++b)
 		{
-			buf[b].gf0 = m_gf0[b].get();
-			buf[b].gf1 = m_gf1[b].get();
+			views[0].buf[b].gf0 = m_gf0[b].get();
+			views[0].buf[b].gf1 = m_gf1[b].get();
 		}
 		if(training)
 		{
 			// NEE records name the training samples their unoccluded contribution is credited to
-			sqs[0].t = m_st[0].get();
-			sqs[1].t = m_st[1].get();
+			views[0].sqs[0].t = m_st[0].get();
+			views[0].sqs[1].t = m_st[1].get();
 		}
 		gargs.map = m_gmap.get();
 		gargs.feat = m_gfeat.get();
@@ -2607,47 +2660,49 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 		}
 	}
 
-	// The launches of one iteration at position q of the period (path buffer q & 1); `ev`
+	// The launches of one iteration of a wave at position q of the period (path buffer q & 1); `ev`
 	// (optional) brackets each with events.
-	auto iteration = [&](int q, cudaEvent_t* ev)
+	auto iteration = [&](WaveView& x, int q, cudaEvent_t* ev)
 	{
 		const int b = q & 1;
-		const PathBuffers& cur = buf[b];
-		const PathBuffers& nxt = buf[1 - b];
-		RenderCounters* const d_counters = counters_of[b];
+		Wave& w = *x.wave;
+		cudaStream_t const st = w.stream;
+		const PathBuffers& cur = x.buf[b];
+		const PathBuffers& nxt = x.buf[1 - b];
+		RenderCounters* const d_counters = x.counters[b];
 		if(ev) { PG_CUDA_CHECK(cudaEventRecord(ev[0], st)); }
 		if(ev) { PG_CUDA_CHECK(cudaEventRecord(ev[1], st)); }
 		// the training samples of a period start at q = 1
 		const uint32_t pos = training ? static_cast<uint32_t>(q) : 2u;
 		if(multi)
 		{
-			begin_kernel<true><<<grid, kShadeBlock, 0, st>>>(counters_of[1 - b], d_counters, capacity, pos,
-			                                                 train_cap / 4u * 3u, m_dev.cam, film, consts, cur, bview);
+			begin_kernel<true><<<grid, kShadeBlock, 0, st>>>(x.counters[1 - b], d_counters, wave_capacity, pos,
+			                                                 train_cap / 4u * 3u, m_dev.cam, film, x.consts, cur, bview);
 		}
 		else
 		{
-			begin_kernel<false><<<grid, kShadeBlock, 0, st>>>(counters_of[1 - b], d_counters, capacity, pos,
-			                                                  train_cap / 4u * 3u, m_dev.cam, film, consts, cur, bview);
+			begin_kernel<false><<<grid, kShadeBlock, 0, st>>>(x.counters[1 - b], d_counters, wave_capacity, pos,
+			                                                  train_cap / 4u * 3u, m_dev.cam, film, x.consts, cur, bview);
 		}
 		PG_CUDA_CHECK(cudaGetLastError());
 		if(ev) { PG_CUDA_CHECK(cudaEventRecord(ev[2], st)); }
-		const ShadowQueue& sq = sqs[b];   // this iteration's NEE segments
+		const ShadowQueue& sq = x.sqs[b];   // this iteration's NEE segments
 		// closest hits of this iteration and the previous iteration's NEE segments (whose
 		// unoccluded contributions, in a training render, are also credited to training samples)
-		launch_trace(m_dev, d_counters, cur.ray_o, cur.ray_d, m_hits.get(), sqs[1 - b], cur.rad, film, refill, st,
-		             counting, cur.meta, multi ? &bview : nullptr, sqs[1 - b].t ? m_tdirw.get() : nullptr);
+		launch_trace(m_dev, d_counters, cur.ray_o, cur.ray_d, w.hits.get(), x.sqs[1 - b], cur.rad, film, refill, waves > 1u, st,
+		             counting, cur.meta, multi ? &bview : nullptr, x.sqs[1 - b].t ? m_tdirw.get() : nullptr);
 		if(!classify)
 		{
 			// slot order
 		}
 		else if(multi)
 		{
-			classify_kernel<true><<<grid, kShadeBlock, 0, st>>>(m_dev, d_counters, m_hits.get(), m_order.get(),
+			classify_kernel<true><<<grid, kShadeBlock, 0, st>>>(m_dev, d_counters, w.hits.get(), w.order.get(),
 			                                                    m_order_list, cur.meta, bview, 0u);
 		}
 		else
 		{
-			classify_kernel<false><<<grid, kShadeBlock, 0, st>>>(m_dev, d_counters, m_hits.get(), m_order.get(),
+			classify_kernel<false><<<grid, kShadeBlock, 0, st>>>(m_dev, d_counters, w.hits.get(), w.order.get(),
 			                                                     m_order_list, cur.meta, bview, guide_depth);
 		}
 		PG_CUDA_CHECK(cudaGetLastError());
@@ -2656,20 +2711,20 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 		if(guided)
 		{
 			// network inputs of this iteration's guidable vertices, then the tensor-core forward pass
-			guide_query_kernel<<<grid, kShadeBlock, 0, st>>>(m_dev, d_counters, cur, m_hits.get(), gargs_b, guide_depth);
+			guide_query_kernel<<<grid, kShadeBlock, 0, st>>>(m_dev, d_counters, cur, w.hits.get(), gargs_b, guide_depth);
 			PG_CUDA_CHECK(cudaGetLastError());
-			guide::launch_forward(m_gimage.get(), m_gfeat.get(), capacity, nullptr, nullptr, m_gerr.get(), st,
+			guide::launch_forward(m_gimage.get(), m_gfeat.get(), wave_capacity, nullptr, nullptr, m_gerr.get(), st,
 			                      &d_counters->n_guided, m_graw.get());
 		}
 		if(ev) { PG_CUDA_CHECK(cudaEventRecord(ev[4], st)); }
-		ShadeArgs sa{m_dev, cur, nxt, m_hits.get(), sq, d_counters, film, consts, max_bounces, params.estimator,
+		ShadeArgs sa{m_dev, cur, nxt, w.hits.get(), sq, d_counters, film, x.consts, max_bounces, params.estimator,
 		             static_cast<uint32_t>(wh)};
 		sa.guide = gargs_b;
 		sa.refine.mode = params.refine_mode;
 		sa.refine.delta = params.refine_delta;
 		sa.refine.iters = static_cast<int>(params.refine_iters);
-		sa.refine_queue = queue_nee ? RefineQueue{m_req_single.get(), m_req_mutual.get()} : RefineQueue{};
-		sa.order = classify ? m_order.get() : nullptr;
+		sa.refine_queue = queue_nee ? RefineQueue{w.req_single.get(), w.req_mutual.get()} : RefineQueue{};
+		sa.order = classify ? w.order.get() : nullptr;
 		sa.order_capacity = m_order_list;
 		sa.batch = bview;
 		if(multi)
@@ -2748,9 +2803,11 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 	{
 		m_inflight.resize(wh);
 	}
-	auto publish_preview = [&](const RenderCounters& hc)
+	auto publish_preview = [&]
 	{
 		RenderProgress& pr = *params.progress;
+		unsigned long long finished = 0;
+		PathRanges generated{};
 		{
 			std::lock_guard<std::mutex> lock(*pr.mutex);
 			const uint32_t pixels = static_cast<uint32_t>(wh);
@@ -2758,17 +2815,27 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 			if(box)
 			{
 				PG_CUDA_CHECK(cudaMemsetAsync(m_inflight.get(), 0, wh * sizeof(uint32_t), st));
-				count_inflight_kernel<<<grid, kShadeBlock, 0, st>>>(buf[0].path, counters_of[1], pixels, m_inflight.get());
-				PG_CUDA_CHECK(cudaGetLastError());
 			}
-			develop_preview_kernel<<<grid, kShadeBlock, 0, st>>>(film_sums, m_inflight.get(), pixels, params.spp,
-			                                                    hc.next_path, box ? 1 : 0, pr.preview_rgb);
+			for(uint32_t v = 0; v < waves; ++v)
+			{
+				const WaveView& x = views[v];
+				if(box)
+				{
+					count_inflight_kernel<<<grid, kShadeBlock, 0, st>>>(x.buf[0].path, x.counters[1], pixels, m_inflight.get());
+					PG_CUDA_CHECK(cudaGetLastError());
+				}
+				generated.first[v] = x.first;
+				generated.end[v] = x.host->next_path;
+				finished += x.host->next_path - x.first - x.host->n_next;
+			}
+			develop_preview_kernel<<<grid, kShadeBlock, 0, st>>>(film_sums, m_inflight.get(), pixels, params.spp, generated,
+			                                                    box ? 1 : 0, pr.preview_rgb);
 			PG_CUDA_CHECK(cudaGetLastError());
 			PG_CUDA_CHECK(cudaStreamSynchronize(st));
 		}
 		if(pr.published)
 		{
-			pr.published(hc.next_path - hc.n_next, total);
+			pr.published(finished, total);
 		}
 	};
 	for(cudaEvent_t& e : m_events)
@@ -2791,10 +2858,11 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 		// in batches of 4, 8, ... ran up to 14 empty iterations on short renders: a 64 x 48 thumbnail
 		// took 24 iterations for its 9.) The graph is built again only when something its launches
 		// were given has changed.
-		std::vector<uint64_t> key = {static_cast<uint64_t>(period), guided, training, multi, kinds, static_cast<uint64_t>(grid),
-		                             capacity, static_cast<uint64_t>(refill), m_order_list, max_bounces, params.estimator, wh,
+		std::vector<uint64_t> key = {static_cast<uint64_t>(period), waves, guided, training, multi, kinds, static_cast<uint64_t>(grid),
+		                             wave_capacity, static_cast<uint64_t>(refill), m_order_list, max_bounces, params.estimator, wh,
 		                             params.refine_mode, float_bits(params.refine_delta), params.refine_iters,
-		                             m_dev.env_map.exact, guide_depth, train_cap, bview.count, m_buffer_generation, params.filter, queue_nee,
+		                             m_dev.env_map.exact, guide_depth, train_cap, bview.count, m_buffer_generation,
+		                             params.filter, queue_nee,
 		                             reinterpret_cast<uint64_t>(film.sums), reinterpret_cast<uint64_t>(film.samples)};
 		if(guided)
 		{
@@ -2803,41 +2871,73 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 				key.push_back(float_bits(v));
 			}
 		}
-		if(!m_exec || m_exec_key != key)
+		for(uint32_t v = 0; v < waves; ++v)
 		{
-			build_loop_graph([&](cudaGraphConditionalHandle loop)
+			WaveView& x = views[v];
+			if(!x.wave->exec || x.wave->exec_key != key)
 			{
-				for(int q = 0; q < period; ++q)
+				build_loop_graph(*x.wave, [&](cudaGraphConditionalHandle loop)
 				{
-					iteration(q, nullptr);
-				}
-				end_kernel<<<1, 1, 0, st>>>(counters_of[1], loop);
-				PG_CUDA_CHECK(cudaGetLastError());
-			});
-			m_exec_key = key;
-		}
-		PG_CUDA_CHECK(cudaEventRecord(e0, st));
-		add_box_weights();
-		while(!done)
-		{
-			PG_CUDA_CHECK(cudaGraphLaunch(m_exec, st));
-			PG_CUDA_CHECK(cudaMemcpyAsync(host_counters, counters_of[1], kCountersHead, cudaMemcpyDeviceToHost, st));
-			PG_CUDA_CHECK(cudaStreamSynchronize(st));
-			iterations = host_counters->iterations;
-			done = render_done(*host_counters);
-			if(host_counters->error || iterations >= kMaxIterations)
-			{
-				break;
+					for(int q = 0; q < period; ++q)
+					{
+						iteration(x, q, nullptr);
+					}
+					end_kernel<<<1, 1, 0, x.wave->stream>>>(x.counters[1], loop);
+					PG_CUDA_CHECK(cudaGetLastError());
+				});
+				x.wave->exec_key = key;
 			}
-			if(!done)
+		}
+		// (should a call below throw, nothing of this render is left running on the other stream)
+		struct WaitForWaves
+		{
+			Wave* waves;
+			uint32_t count;
+			~WaitForWaves()
+			{
+				for(uint32_t v = 1; v < count; ++v)
+				{
+					cudaStreamSynchronize(waves[v].stream);
+				}
+			}
+		} wait_for_waves{m_waves, waves};
+		PG_CUDA_CHECK(cudaEventRecord(e0, st));
+		for(uint32_t v = 1; v < waves; ++v)
+		{
+			PG_CUDA_CHECK(cudaStreamWaitEvent(m_waves[v].stream, e0));   // the uploads
+		}
+		add_box_weights();
+		bool failed = false;
+		while(!done && !failed)
+		{
+			for(uint32_t v = 0; v < waves; ++v)
+			{
+				WaveView& x = views[v];
+				if(!x.done)
+				{
+					PG_CUDA_CHECK(cudaGraphLaunch(x.wave->exec, x.wave->stream));
+					PG_CUDA_CHECK(cudaMemcpyAsync(x.host, x.counters[1], kCountersHead, cudaMemcpyDeviceToHost, x.wave->stream));
+				}
+			}
+			done = true;
+			for(uint32_t v = 0; v < waves; ++v)
+			{
+				WaveView& x = views[v];
+				PG_CUDA_CHECK(cudaStreamSynchronize(x.wave->stream));
+				x.done = render_done(*x.host);
+				done = done && x.done;
+				failed = failed || x.host->error || x.host->iterations >= kMaxIterations;
+			}
+			if(!done && !failed)
 			{
 				if(!params.progress)
 				{
 					break;   // only progress points end the loop before the last path
 				}
-				publish_preview(*host_counters);
+				publish_preview();
 			}
 		}
+		done = done && !failed;
 		splat_samples();
 		PG_CUDA_CHECK(cudaEventRecord(e1, st));
 		PG_CUDA_CHECK(cudaEventSynchronize(e1));
@@ -2854,9 +2954,9 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 		while(!done && iterations < kMaxIterations)
 		{
 			const int q = static_cast<int>(iterations % static_cast<unsigned long long>(period));
-			iteration(q, timing ? ev : nullptr);
+			iteration(views[0], q, timing ? ev : nullptr);
 			++iterations;
-			PG_CUDA_CHECK(cudaMemcpyAsync(host_counters, counters_of[q & 1], kCountersHead, cudaMemcpyDeviceToHost, st));
+			PG_CUDA_CHECK(cudaMemcpyAsync(views[0].host, views[0].counters[q & 1], kCountersHead, cudaMemcpyDeviceToHost, st));
 			PG_CUDA_CHECK(cudaStreamSynchronize(st));
 			if(timing)
 			{
@@ -2869,8 +2969,8 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 					m_kernel_ms[slot[k]] += ms;
 				}
 			}
-			done = render_done(*host_counters);
-			if(host_counters->error)
+			done = render_done(*views[0].host);
+			if(views[0].host->error)
 			{
 				break;
 			}
@@ -2883,8 +2983,17 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 
 	float ms = 0.0f;
 	PG_CUDA_CHECK(cudaEventElapsedTime(&ms, e0, e1));
-	const RenderCounters final_counters = *host_counters;
-
+	// the waves' counts together
+	RenderCounters final_counters = *views[0].host;
+	for(uint32_t v = 1; v < waves; ++v)
+	{
+		const RenderCounters& c = *views[v].host;
+		final_counters.rays_traced += c.rays_traced;
+		final_counters.shadow_rays += c.shadow_rays;
+		final_counters.iterations += c.iterations;
+		final_counters.error |= c.error;
+	}
+	iterations = final_counters.iterations;
 	m_last_rays = final_counters.rays_traced;
 	m_last_shadow = final_counters.shadow_rays;
 	m_last_iterations = iterations;

@@ -348,12 +348,13 @@ constexpr uint32_t kTargetFinal = 0x80000000u;
 // Launcher implemented in pg_trace.cu (FMA-enabled traversal kernels); min_idle is the
 // traversal's refill threshold (LaunchConfig::refill). Closest hits of this iteration's queue and visibility of the previous iteration's shadow
 // queue `prev` in one persistent launch; unoccluded contributions go to rad_cur / the film.
+// shared: another wavefront's kernels run beside it.
 // With a batch (multi-scene render), `meta` is the current path buffer's meta words and prev.sid
 // the records' scenes. With train_dirw (guided training renders), an unoccluded record whose
 // prev.t names a training sample adds its weight to that sample.
 void launch_trace(const DeviceScene& s, RenderCounters* counters, const float4* ray_o, const float4* ray_d,
                   uint2* hits, const ShadowQueue& prev, float4* rad_cur, const FilmView& film, int min_idle,
-                  cudaStream_t st, bool count, const uint32_t* meta = nullptr, const BatchView* batch = nullptr,
+                  bool shared, cudaStream_t st, bool count, const uint32_t* meta = nullptr, const BatchView* batch = nullptr,
                   float4* train_dirw = nullptr);
 
 // A scene resident on the GPU together with its render buffers.
@@ -434,8 +435,9 @@ public:
 
 private:
 	float render_pass(const RenderParams& params, double* film_device, const std::vector<BatchScene>* batch = nullptr);
-	void ensure_capacity(uint32_t capacity, uint32_t grid);
-	void build_loop_graph(const std::function<void(cudaGraphConditionalHandle)>& launches);
+	struct Wave;
+	void ensure_capacity(uint32_t waves, uint32_t capacity, uint32_t grid);
+	void build_loop_graph(Wave& wave, const std::function<void(cudaGraphConditionalHandle)>& launches);
 	// Coordinate descent over the launch shapes (pool depth, refill threshold, blocks per SM, and
 	// optionally leaf size), `measure` giving a candidate's calibration milliseconds; the winner is
 	// set on this scene.
@@ -453,28 +455,41 @@ private:
 	DeviceBuffer<float2>      m_env_alias;
 	DeviceScene               m_dev{};
 
-	uint32_t m_capacity = 0;
+	uint32_t m_capacity = 0;   // path slots of each wave
 	uint32_t m_order_grid = 0;
 	LaunchConfig m_launch;
 	float m_max_origin_abs = 0.0f;
 	uint32_t m_bvh_builder = 0;
 	std::vector<uint32_t> m_material_types;   // per material (fingerprint)
 	uint32_t m_shade_kinds = 0;               // bit per shading kernel the materials need besides the matte one
-	// the path pool: one allocation, carved by ensure_capacity
-	DeviceBuffer<unsigned char> m_pool;
-	DeviceSpan<uint32_t> m_path[2], m_meta[2];
-	DeviceSpan<float4>   m_thr[2], m_rad[2], m_prev[2], m_ro[2], m_rd[2];
-	DeviceSpan<uint2>    m_hits;
-	DeviceSpan<float4>   m_so[2], m_sd[2], m_sc[2];   // shadow queues, one per iteration parity
-	DeviceSpan<float2>   m_sr[2];
-	DeviceSpan<uint32_t> m_req_single, m_req_mutual;
-	DeviceSpan<uint32_t> m_order;   // shading order: kOrderLists lists of m_order_list slots
+	// One of the wavefronts a render runs: its own part of the path pool, counters, stream and loop
+	// graph. Renders of many paths run two side by side (render_pass).
+	struct Wave
+	{
+		cudaStream_t stream = nullptr;   // the first wave's is m_stream
+		DeviceSpan<uint32_t> path[2], meta[2];
+		DeviceSpan<float4>   thr[2], rad[2], prev[2], ro[2], rd[2];
+		DeviceSpan<uint2>    hits;
+		DeviceSpan<float4>   so[2], sd[2], sc[2];   // shadow queues, one per iteration parity
+		DeviceSpan<float2>   sr[2];
+		DeviceSpan<uint32_t> sid[2];                // multi-scene renders: scene of each NEE record
+		DeviceSpan<uint32_t> req_single, req_mutual;
+		DeviceSpan<uint32_t> order;                 // shading order: kOrderLists lists of m_order_list slots
+		DeviceBuffer<RenderState> state;
+		RenderState* host_state = nullptr;          // pinned staging of `state`
+		// the instantiated loop graph of the last render with everything its launches were given (kept
+		// across renders)
+		cudaGraphExec_t exec = nullptr;
+		std::vector<uint64_t> exec_key;
+	};
+	static constexpr uint32_t kMaxWaves = 2;
+	Wave m_waves[kMaxWaves];
+	DeviceBuffer<unsigned char> m_pool;   // the waves' buffers: one allocation, carved by ensure_capacity
+	uint32_t m_pool_waves = 0;
 	DeviceBuffer<float4>   m_samples; // 4 x 4 filters: radiance of every path of a pass
 	DeviceBuffer<uint32_t> m_inflight;   // previews: paths in flight per pixel
-	DeviceBuffer<uint32_t> m_ssid[2];    // multi-scene renders: scene of each NEE record
 	DeviceBuffer<BatchScene> m_batch_table;
 	uint32_t m_order_list = 0;
-	DeviceBuffer<RenderState> m_state;
 
 	// learned guiding
 	GuideParams m_guide_params;
@@ -496,12 +511,7 @@ private:
 
 	// the scene's own stream: renders of different scenes, from different host threads, overlap
 	cudaStream_t m_stream = nullptr;
-	// pinned staging of m_state, the render's two timing events, and the instantiated loop graph of the
-	// last render with everything its launches were given (kept across renders)
-	RenderState* m_host_state = nullptr;
-	cudaEvent_t m_events[2] = {nullptr, nullptr};
-	cudaGraphExec_t m_exec = nullptr;
-	std::vector<uint64_t> m_exec_key;
+	cudaEvent_t m_events[2] = {nullptr, nullptr};   // a render's timing
 	uint64_t m_buffer_generation = 0;   // counts reallocations of buffers that a graph's launches name
 
 	unsigned long long m_last_rays = 0, m_last_shadow = 0, m_last_iterations = 0, m_last_launches = 0;

@@ -359,33 +359,36 @@ trace_kernel(const WideNode* __restrict__ nodes, const LeafTri* __restrict__ tri
 
 void launch_trace(const DeviceScene& s, RenderCounters* counters, const float4* ray_o, const float4* ray_d,
                   uint2* hits, const ShadowQueue& prev, float4* rad_cur, const FilmView& film, int min_idle,
-                  cudaStream_t st, bool count, const uint32_t* meta, const BatchView* batch, float4* train_dirw)
+                  bool shared, cudaStream_t st, bool count, const uint32_t* meta, const BatchView* batch, float4* train_dirw)
 {
+	// beside another wavefront, one block per SM less: the room it leaves lets the other's kernels in while
+	// this one runs (6 and 7 blocks of 8 measured alike, 8 without gain)
+	const int left_free = shared ? sm_count() : 0;
 	if(batch)
 	{
 		if(count)
 		{
-			const int grid = persistent_grid(trace_kernel<true, true>);
+			const int grid = std::max(1, persistent_grid(trace_kernel<true, true>) - left_free);
 			trace_kernel<true, true><<<grid, kTraceBlock, 0, st>>>(s.nodes, s.tris, counters, ray_o, ray_d, hits,
 				prev.o, prev.d, prev.c, prev.r, rad_cur, film, min_idle, meta, prev.sid, *batch, nullptr, nullptr);
 		}
 		else
 		{
-			const int grid = persistent_grid(trace_kernel<false, true>);
+			const int grid = std::max(1, persistent_grid(trace_kernel<false, true>) - left_free);
 			trace_kernel<false, true><<<grid, kTraceBlock, 0, st>>>(s.nodes, s.tris, counters, ray_o, ray_d, hits,
 				prev.o, prev.d, prev.c, prev.r, rad_cur, film, min_idle, meta, prev.sid, *batch, nullptr, nullptr);
 		}
 	}
 	else if(count)
 	{
-		const int grid = persistent_grid(trace_kernel<true, false>);
+		const int grid = std::max(1, persistent_grid(trace_kernel<true, false>) - left_free);
 		trace_kernel<true, false><<<grid, kTraceBlock, 0, st>>>(s.nodes, s.tris, counters, ray_o, ray_d, hits,
 			prev.o, prev.d, prev.c, prev.r, rad_cur, film, min_idle, nullptr, nullptr, BatchView{},
 			train_dirw ? prev.t : nullptr, train_dirw);
 	}
 	else
 	{
-		const int grid = persistent_grid(trace_kernel<false, false>);
+		const int grid = std::max(1, persistent_grid(trace_kernel<false, false>) - left_free);
 		trace_kernel<false, false><<<grid, kTraceBlock, 0, st>>>(s.nodes, s.tris, counters, ray_o, ray_d, hits,
 			prev.o, prev.d, prev.c, prev.r, rad_cur, film, min_idle, nullptr, nullptr, BatchView{},
 			train_dirw ? prev.t : nullptr, train_dirw);

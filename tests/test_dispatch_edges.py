@@ -142,3 +142,24 @@ def test_graph_reuse_gives_a_fresh_scenes_film(gpu_lib):
         with photon_gpu.RenderScene(scene) as fresh:
             fresh.render(**shapes[0])
             np.testing.assert_allclose(used.film()[1], fresh.film()[1], rtol=1e-11, atol=0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sample_filter", ["box", "bh"])
+@pytest.mark.parametrize("width,height,spp", [(32, 32, 1), (32, 32, 2), (33, 31, 2), (45, 23, 5), (64, 33, 7)])
+def test_two_wavefronts_give_one_wavefronts_film(gpu_lib, sample_filter, width, height, spp):
+    """Renders of at least two pools of paths run as two wavefronts: pools of 1,024 paths (the smallest)
+    against one that holds them all, and the ray counts."""
+    import photon_gpu
+
+    scene = scenes.cornell_glossy(width, height, spp, 8)
+    films, rays = [], []
+    for capacity in (1024, 1 << 20):
+        with photon_gpu.RenderScene(scene) as rs:
+            rs.set_launch(capacity=capacity)
+            rs.set_filter(sample_filter)
+            r = rs.render(spp, max_bounces=8, seed=21)
+            films.append(rs.film()[1])
+            rays.append((r["rays"], r["shadow_rays"]))
+    assert rays[0] == rays[1]
+    np.testing.assert_allclose(films[0], films[1], rtol=1e-11, atol=1e-11 * np.abs(films[1]).max())
