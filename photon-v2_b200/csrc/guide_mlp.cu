@@ -4,10 +4,11 @@
 // One CTA per SM, of kTeams teams of 256 threads that share the weights in shared memory; each team
 // walks 128-row tiles of queries on its own (its barriers are named, its accumulator and mbarrier its
 // own). A tile is a chain of dependent MMA groups and per-row work, so the tiles in flight on an SM are
-// what hides its latency: three teams instead of two one-team CTAs took a 192-sample guided Cornell
-// render from 19.85 to 19.0 ms; two teams were as slow as the two CTAs, a fourth gave no more. Each row
-// is owned by two threads (part 0: threads 0-127, part 1: threads 128-255, thread t and t + 128 on row
-// t), so that the per-row work between the MMAs is split in two.
+// what hides its latency: 1 M queries with their mixtures took 400 us with two one-team CTAs per SM,
+// 312 us with three teams, 286 us with the rows' BF16 conversions paired (one at a time, they kept half
+// of their pipe busy), 266 us with four teams and the next tile's inputs loaded during the layers. Each
+// row is owned by two threads (part 0: threads 0-127, part 1: threads 128-255, thread t and t + 128 on
+// row t), so that the per-row work between the MMAs is split in two.
 // Per tile:
 //   1. the two threads of a row one-blob encode its inputs (alternating inputs) into the A
 //      operand buffer (BF16, 224 columns, fed to the MMAs in two K halves);
@@ -49,7 +50,7 @@ using namespace tc;
 
 constexpr int kTeamThreads = 256;             // two threads per tile row
 constexpr int kParts = kTeamThreads / kTile;
-constexpr int kTeams = 3;
+constexpr int kTeams = 4;
 constexpr int kThreads = kTeams * kTeamThreads;
 constexpr uint32_t kTmemCols = 256;   // power of two >= 64 accumulator columns per team
 static_assert(kTeams * kHidden <= static_cast<int>(kTmemCols), "tensor memory");
@@ -154,18 +155,22 @@ mlp_forward_kernel(const unsigned char* __restrict__ image, const float* __restr
 	uint32_t phase = 0;
 	bool failed = false;
 	const uint32_t num_tiles = (n + kTile - 1) / kTile;
+	// a row's inputs (two 16-byte loads)
+	float f[kInputs];
+	auto load_inputs = [&](uint32_t row)
+	{
+		const float4* src = reinterpret_cast<const float4*>(features) + static_cast<size_t>(row) * 2;
+		const float4 none = make_float4(-1.0f, -1.0f, -1.0f, -1.0f);
+		const float4 a = row < n ? __ldg(src) : none, b = row < n ? __ldg(src + 1) : none;
+		f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w;
+		f[4] = b.x; f[5] = b.y; f[6] = b.z;
+	};
+	load_inputs((team * gridDim.x + blockIdx.x) * kTile + r);
 	// (a team's first tile is gridDim.x after the previous team's, so that few tiles spread over the SMs)
 	for(uint32_t tile = team * gridDim.x + blockIdx.x; tile < num_tiles && !failed; tile += kTeams * gridDim.x)
 	{
 		const uint32_t row = tile * kTile + r;
 		const bool valid = row < n;
-
-		float f[kInputs];
-		#pragma unroll
-		for(int i = 0; i < kInputs; ++i)
-		{
-			f[i] = valid ? __ldg(features + static_cast<size_t>(row) * 8 + i) : -1.0f;
-		}
 
 		// One MMA chain (k_steps x K = 16) from the team's A buffer against weights w_base starting at
 		// global K-step ks0, committed to the mbarrier; every thread then waits for it.
@@ -252,6 +257,8 @@ mlp_forward_kernel(const unsigned char* __restrict__ image, const float* __restr
 			failed = true;
 			break;
 		}
+
+		load_inputs((tile + kTeams * gridDim.x) * kTile + r);   // the next tile's, in flight during the layers
 
 		// 2./3. H1 -> H2 -> H3 -> H4 -> out
 		#pragma unroll 1

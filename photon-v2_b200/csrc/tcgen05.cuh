@@ -116,13 +116,13 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v)
 
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// Two floats rounded to BF16 by one conversion, a in the low half.
 __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b)
 {
-	const __nv_bfloat16 lo = __float2bfloat16_rn(a);
-	const __nv_bfloat16 hi = __float2bfloat16_rn(b);
-	return static_cast<uint32_t>(__bfloat16_as_ushort(lo)) | (static_cast<uint32_t>(__bfloat16_as_ushort(hi)) << 16);
+	uint32_t d;
+	asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(b), "f"(a));
+	return d;
 }
-
 
 }// end namespace tc
 }// end namespace pg
