@@ -492,12 +492,7 @@ void launch_forward(const unsigned char* d_image, const float* d_features, uint3
 	{
 		return;
 	}
-	static const bool configured = []
-	{
-		PG_CUDA_CHECK(cudaFuncSetAttribute(mlp_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-		return true;
-	}();
-	(void)configured;
+	allow_shared_memory(reinterpret_cast<const void*>(mlp_forward_kernel), kSmemBytes);
 	const uint32_t tiles = (n + kTile - 1) / kTile;
 	const uint32_t grid = std::min<uint32_t>(tiles, static_cast<uint32_t>(sm_count()));
 	mlp_forward_kernel<<<grid, kThreads, kSmemBytes, s>>>(d_image, d_features, n, d_n, d_out_raw, d_out_mix,

@@ -876,13 +876,7 @@ void launch_gradients(const float* d_params, const unsigned char* d_image, const
 	launch_forward(d_image, d_features, n, d_raw, d_acts, d_error, s, d_n);
 	if(tensor_cores)
 	{
-		static const bool configured_tc = []
-		{
-			PG_CUDA_CHECK(cudaFuncSetAttribute(tcb::backward_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-			                                   tcb::kSmemBytes));
-			return true;
-		}();
-		(void)configured_tc;
+		allow_shared_memory(reinterpret_cast<const void*>(tcb::backward_tc_kernel), tcb::kSmemBytes);
 		const uint32_t grid = backward_grid(n);
 		tcb::backward_tc_kernel<<<grid, tcb::kThreads, tcb::kSmemBytes, s>>>(d_params, d_features, d_dirw, d_raw, d_acts,
 		                                                                     n, d_n, d_total, d_partials, d_loss, d_error);
@@ -895,12 +889,7 @@ void launch_gradients(const float* d_params, const unsigned char* d_image, const
 		return;
 	}
 	constexpr int smem_bytes = 2 * kBlock * kPitch * sizeof(float);
-	static const bool configured = []
-	{
-		PG_CUDA_CHECK(cudaFuncSetAttribute(backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
-		return true;
-	}();
-	(void)configured;
+	allow_shared_memory(reinterpret_cast<const void*>(backward_kernel), smem_bytes);
 	backward_kernel<<<(n + kBlock - 1) / kBlock, kBlock, smem_bytes, s>>>(d_params, d_features, d_dirw, d_raw, d_acts,
 	                                                                     n, d_n, d_total, d_grads, d_loss);
 	PG_CUDA_CHECK(cudaGetLastError());

@@ -351,12 +351,7 @@ void launch_film_samples(const FilmView& film, uint64_t seed, uint64_t first_glo
 		PG_CUDA_CHECK(cudaGetLastError());
 		return;
 	}
-	static const bool configured = []
-	{
-		PG_CUDA_CHECK(cudaFuncSetAttribute(gather_samples_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGatherSmem));
-		return true;
-	}();
-	(void)configured;
+	allow_shared_memory(reinterpret_cast<const void*>(gather_samples_kernel), kGatherSmem);
 	const uint32_t tx = (film.width + kGatherX - 1u) / kGatherX, ty = (film.height + kGatherY - 1u) / kGatherY;
 	// three blocks fit an SM; several rounds of them keep the last one short
 	const uint32_t split = std::min<uint32_t>(spp, std::max<uint32_t>(1u, 12u * static_cast<uint32_t>(sms) / (tx * ty)));

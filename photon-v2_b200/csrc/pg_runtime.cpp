@@ -1,6 +1,8 @@
 #include "pg_runtime.h"
 
 #include <mutex>
+#include <set>
+#include <utility>
 
 namespace pg
 {
@@ -153,6 +155,19 @@ void check_same_device(int owner_device, int current, const char* what)
 void require_same_device(int owner_device, const char* what)
 {
 	check_same_device(owner_device, current_device(), what);
+}
+
+void allow_shared_memory(const void* kernel, int bytes)
+{
+	static std::mutex mutex;
+	static std::set<std::pair<const void*, int>> allowed;
+	const auto key = std::make_pair(kernel, current_device());
+	std::lock_guard<std::mutex> lock(mutex);
+	if(allowed.count(key) == 0)
+	{
+		PG_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+		allowed.insert(key);
+	}
 }
 
 int sm_count()

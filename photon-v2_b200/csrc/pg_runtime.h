@@ -248,6 +248,10 @@ private:
 constexpr std::size_t kPinnedStage = std::size_t(256) << 10;
 unsigned char* pinned_stage();
 
+// Lets a kernel use `bytes` of dynamic shared memory on the current device (above 48 KB that has to be
+// asked for, once per kernel and device).
+void allow_shared_memory(const void* kernel, int bytes);
+
 // Number of SMs of the current device (grid sizing).
 int sm_count();
 
