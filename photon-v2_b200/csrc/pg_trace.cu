@@ -48,6 +48,10 @@ constexpr int kTraceBlock = kTraversalBlock;
 // Resident blocks per SM the traversal kernels are compiled for: 8 x 128 threads at 64 registers
 // fill the register file (a larger register budget leaves room for 7 blocks only).
 constexpr int kTraceMinBlocks = 8;
+// Rays of several scenes carry their tree's two addresses, which do not fit 64 registers (100 bytes of
+// spills): 72 registers at seven blocks. Eight scenes at 1/8 of their samples in one wavefront: 102.0 ms
+// a call with eight blocks, 98.2 with seven, 104.3 with six.
+constexpr int kTraceMinBlocksMulti = 7;
 
 struct HitRecord
 {
@@ -271,7 +275,7 @@ __device__ __forceinline__ void add_unoccluded(uint32_t i, const float4* __restr
 // path's meta word, a NEE segment's in its record's sid); each ray walks its own scene's tree and
 // a final contribution goes to its own scene's film.
 template<bool COUNT, bool MULTI>
-__global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks)
+__global__ void __launch_bounds__(kTraceBlock, MULTI ? kTraceMinBlocksMulti : kTraceMinBlocks)
 trace_kernel(const WideNode* __restrict__ nodes, const LeafTri* __restrict__ tris,
              RenderCounters* __restrict__ counters,
              const float4* __restrict__ ray_o, const float4* __restrict__ ray_d, uint2* __restrict__ hits,
