@@ -176,7 +176,7 @@ __device__ __forceinline__ void splat(const FilmView& f, uint32_t pixel, uint32_
 	}
 	else
 	{
-		f.samples[path] = make_float4(c.r, c.g, c.b, 0.0f);   // splatted by splat_samples_kernel
+		f.samples[path] = make_float4(c.r, c.g, c.b, 0.0f);   // into the film at the end of the pass (launch_film_samples)
 	}
 }
 
@@ -425,7 +425,7 @@ __device__ __forceinline__ bool guidable(const Material& m)
 	return m.type == PG_MAT_MATTE && (m.cr > 0.0f || m.cg > 0.0f || m.cb > 0.0f);
 }
 
-// Whether guide_query_kernel gives the queue entry a network row: a hit on a guidable surface at
+// Whether classify_kernel lists a hit as a guided vertex: on a guidable surface at
 // a vertex below the guiding depth, on a path that continues after it.
 __device__ __forceinline__ bool guided_vertex(const Material& m, uint32_t meta, uint32_t guide_depth)
 {
@@ -677,43 +677,88 @@ __device__ __noinline__ V3 guide_sample(const float* __restrict__ mix, float u0,
 	return guide::vmf_sample(v3(a.y, b.x, b.y), c.x, u1, u2);
 }
 
-// Network inputs for every queue entry that will be shaded at a guidable vertex; entries are
-// compacted into rows (map: entry -> row).
-__global__ void __launch_bounds__(kShadeBlock)
-guide_query_kernel(DeviceScene s, RenderCounters* __restrict__ c, PathBuffers cur, const uint2* __restrict__ hits,
-                   GuideArgs g, uint32_t max_bounces)
+// The slots of LISTS neighbouring class lists, numbered through list by list (class-major).
+template<uint32_t LISTS>
+struct ClassItems
 {
-	const uint32_t total = c->n_total;
-	for(uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x)
+	uint32_t end[LISTS];   // the number of slots up to the end of each list
+
+	// One warp sums up the list lengths (one thread loading them one after another took longer than
+	// shading a small queue).
+	__device__ __forceinline__ void fill(const RenderCounters* c, uint32_t first_list)
 	{
-		const uint2 hit = hits[i];
-		const uint32_t meta = cur.meta[i];
-		uint32_t row = 0xFFFFFFFFu;
-		if(hit.x != 0xFFFFFFFFu)
+		if(threadIdx.x < 32u)
 		{
-			const LeafTri& lt = s.tris[hit.x];
-			if(guided_vertex(s.materials[lt.material], meta, max_bounces))
+			uint32_t before = 0;
+			#pragma unroll
+			for(uint32_t l0 = 0; l0 < LISTS; l0 += 32u)
 			{
-				const float4 o = cur.ray_o[i];
-				const float4 d4 = cur.ray_d[i];
-				const V3 d = v3(d4.x, d4.y, d4.z);
-				const float t = __uint_as_float(hit.y);
-				const V3 pos = v3(o.x, o.y, o.z) + d * t;
-				const V3 a = v3(lt.v0x, lt.v0y, lt.v0z), b = v3(lt.v1x, lt.v1y, lt.v1z), cc = v3(lt.v2x, lt.v2y, lt.v2z);
-				V3 n = normalize(cross(b - a, cc - a));
-				if(dot(n, d) > 0.0f)
+				const uint32_t l = l0 + threadIdx.x;
+				uint32_t e = l < LISTS ? c->n_class[first_list + l].n : 0u;
+				#pragma unroll
+				for(uint32_t d = 1; d < 32u; d *= 2u)
 				{
-					n = -n;   // the side the path arrives on
+					const uint32_t up = __shfl_up_sync(0xFFFFFFFFu, e, d);
+					e += threadIdx.x >= d ? up : 0u;
 				}
-				const guide::Features f = guide::make_features(pos, v3(g.lo[0], g.lo[1], g.lo[2]),
-				                                               v3(g.rcp[0], g.rcp[1], g.rcp[2]), n, -d);
-				row = alloc_slot(&c->n_guided);
-				float4* dst = reinterpret_cast<float4*>(g.feat + static_cast<size_t>(row) * 8);
-				dst[0] = make_float4(f.v[0], f.v[1], f.v[2], f.v[3]);
-				dst[1] = make_float4(f.v[4], f.v[5], f.v[6], 0.0f);
+				e += before;
+				if(l < LISTS)
+				{
+					end[l] = e;
+				}
+				before = __shfl_sync(0xFFFFFFFFu, e, 31);
 			}
 		}
-		g.map[i] = row;
+	}
+	__device__ __forceinline__ uint32_t total() const { return end[LISTS - 1u]; }
+	// The slot of item w: in the first list whose end exceeds w.
+	__device__ __forceinline__ uint32_t slot(uint32_t w, const uint32_t* order, uint32_t list_capacity, uint32_t first_list) const
+	{
+		uint32_t lo = 0, hi = LISTS - 1u;
+		while(lo < hi)
+		{
+			const uint32_t mid = (lo + hi) >> 1;
+			if(w < end[mid]) { hi = mid; } else { lo = mid + 1u; }
+		}
+		return order[(first_list + lo) * list_capacity + (w - (lo ? end[lo - 1u] : 0u))];
+	}
+};
+
+// Network inputs of the vertices that will be guided: one row per item of their class.
+__global__ void __launch_bounds__(kShadeBlock)
+guide_query_kernel(DeviceScene s, RenderCounters* __restrict__ c, PathBuffers cur, const uint2* __restrict__ hits,
+                   GuideArgs g, const uint32_t* __restrict__ order, uint32_t order_capacity)
+{
+	constexpr uint32_t kFirstList = kClassGuided * kClassLists;
+	__shared__ ClassItems<kClassLists> items;
+	items.fill(c, kFirstList);
+	__syncthreads();
+	const uint32_t total = items.total();
+	if(blockIdx.x == 0 && threadIdx.x == 0)
+	{
+		c->n_guided = total;
+	}
+	for(uint32_t row = blockIdx.x * blockDim.x + threadIdx.x; row < total; row += gridDim.x * blockDim.x)
+	{
+		const uint32_t i = items.slot(row, order, order_capacity, kFirstList);
+		const uint2 hit = hits[i];
+		const LeafTri& lt = s.tris[hit.x];
+		const float4 o = cur.ray_o[i];
+		const float4 d4 = cur.ray_d[i];
+		const V3 d = v3(d4.x, d4.y, d4.z);
+		const float t = __uint_as_float(hit.y);
+		const V3 pos = v3(o.x, o.y, o.z) + d * t;
+		const V3 a = v3(lt.v0x, lt.v0y, lt.v0z), b = v3(lt.v1x, lt.v1y, lt.v1z), cc = v3(lt.v2x, lt.v2y, lt.v2z);
+		V3 n = normalize(cross(b - a, cc - a));
+		if(dot(n, d) > 0.0f)
+		{
+			n = -n;   // the side the path arrives on
+		}
+		const guide::Features f = guide::make_features(pos, v3(g.lo[0], g.lo[1], g.lo[2]),
+		                                               v3(g.rcp[0], g.rcp[1], g.rcp[2]), n, -d);
+		float4* dst = reinterpret_cast<float4*>(g.feat + static_cast<size_t>(row) * 8);
+		dst[0] = make_float4(f.v[0], f.v[1], f.v[2], f.v[3]);
+		dst[1] = make_float4(f.v[4], f.v[5], f.v[6], 0.0f);
 	}
 }
 
@@ -759,10 +804,14 @@ __device__ __forceinline__ float4 cur_gf1(const ShadeArgs& a, uint32_t i) { retu
 // instruction fetch.)
 enum ShadeKind : int
 {
-	kShadeMatte = 0,        // misses, light surfaces, matte and guided vertices
+	kShadeMatte = 0,        // misses, light surfaces and matte vertices
 	kShadeConductor = 1,
 	kShadeDielectric = 2,
+	kShadeGuided = 3,       // matte vertices of a guided render that sample the learned mixture
 };
+// (Guided vertices within the matte kernel made it spill 156 bytes a thread: a 256 x 256 guided Cornell
+// box at 192 samples took 17.9 ms a render, with a kernel of their own 17.2; that kernel at 6 or 5 blocks
+// per SM instead of 8: 17.9 and 17.6.)
 
 // GUIDED instantiates the learned-guiding paths; the plain estimator compiles without them.
 // MULTI: each path shades in the scene of its meta word's top bits (a.batch), into that scene's
@@ -771,57 +820,27 @@ template<bool GUIDED, bool MULTI, int KIND>
 __global__ void __launch_bounds__(kShadeBlock, kShadeMinBlocks)
 shade_kernel(ShadeArgs a)
 {
-	constexpr uint32_t kFirstList = (KIND == kShadeMatte ? kClassMiss
+	constexpr bool kMatte = KIND == kShadeMatte || KIND == kShadeGuided;
+	constexpr uint32_t kFirstList = (KIND == kShadeMatte ? kClassMiss : KIND == kShadeGuided ? kClassGuided
 	                                 : KIND == kShadeConductor ? kClassConductor : kClassDielectric) * kClassLists;
-	constexpr uint32_t kLists = (KIND == kShadeMatte ? 4u : 1u) * kClassLists;
-	// work item w -> queue slot: list by list (class-major) through the lists classify_kernel made.
-	// One warp sums up the list lengths (one thread loading them one after another took longer than
-	// shading a small queue).
-	__shared__ uint32_t list_end[kLists];
+	constexpr uint32_t kLists = (KIND == kShadeMatte ? 3u : 1u) * kClassLists;
+	// work item w -> queue slot, through the lists classify_kernel made
+	__shared__ ClassItems<kLists> items;
 	// (once per block: the loop over the items would load these from global memory for every item)
 	__shared__ RenderConsts consts;
 	if(threadIdx.x == 0)
 	{
 		consts = *a.consts;
 	}
-	if(a.order && threadIdx.x < 32u)
+	if(a.order)
 	{
-		uint32_t before = 0;
-		#pragma unroll
-		for(uint32_t l0 = 0; l0 < kLists; l0 += 32u)
-		{
-			const uint32_t l = l0 + threadIdx.x;
-			uint32_t end = l < kLists ? a.counters->n_class[kFirstList + l].n : 0u;
-			#pragma unroll
-			for(uint32_t d = 1; d < 32u; d *= 2u)
-			{
-				const uint32_t up = __shfl_up_sync(0xFFFFFFFFu, end, d);
-				end += threadIdx.x >= d ? up : 0u;
-			}
-			end += before;
-			if(l < kLists)
-			{
-				list_end[l] = end;
-			}
-			before = __shfl_sync(0xFFFFFFFFu, end, 31);
-		}
+		items.fill(a.counters, kFirstList);
 	}
 	__syncthreads();
-	const uint32_t total = a.order ? list_end[kLists - 1u] : a.counters->n_total;
+	const uint32_t total = a.order ? items.total() : a.counters->n_total;
 	for(uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < total; w += gridDim.x * blockDim.x)
 	{
-		uint32_t i = w;
-		if(a.order)
-		{
-			// first list whose end exceeds w
-			uint32_t lo = 0, hi = kLists - 1u;
-			while(lo < hi)
-			{
-				const uint32_t mid = (lo + hi) >> 1;
-				if(w < list_end[mid]) { hi = mid; } else { lo = mid + 1u; }
-			}
-			i = a.order[(kFirstList + lo) * a.order_capacity + (w - (lo ? list_end[lo - 1u] : 0u))];
-		}
+		const uint32_t i = a.order ? items.slot(w, a.order, a.order_capacity, kFirstList) : w;
 		const uint32_t p = a.cur.path[i];
 		const uint32_t meta = a.cur.meta[i];
 		const uint32_t bounce = meta & kMetaBounceMask;
@@ -1021,7 +1040,7 @@ shade_kernel(ShadeArgs a)
 		}
 		Material mat = s.materials[mat_index];
 		const bool absorber = KIND == kShadeMatte && mat.type == PG_MAT_ABSORBER;
-		mat.type = KIND == kShadeMatte ? PG_MAT_MATTE : KIND == kShadeConductor ? PG_MAT_CONDUCTOR : PG_MAT_DIELECTRIC;
+		mat.type = kMatte ? PG_MAT_MATTE : KIND == kShadeConductor ? PG_MAT_CONDUCTOR : PG_MAT_DIELECTRIC;
 		const V3 v = -d;
 
 		// ---- next-event estimation (TDirectLightEstimator::neeSampleEmission,
@@ -1036,14 +1055,14 @@ shade_kernel(ShadeArgs a)
 		RGB sh_c{};
 		uint32_t nee_row = 0xFFFFFFFFu;   // this vertex's NEE direction as a training sample of its own
 		float nee_w = 0.0f;
-		const uint32_t grow = GUIDED && KIND == kShadeMatte ? a.guide.map[i] : 0xFFFFFFFFu;
-		const bool guided = GUIDED && KIND == kShadeMatte && grow != 0xFFFFFFFFu;
+		const uint32_t grow = w;   // a guided vertex' row
+		constexpr bool guided = KIND == kShadeGuided;
 		const float* graw = guided ? a.guide.raw + static_cast<size_t>(grow) * guide::kMixFloats : nullptr;
 		const float alpha = a.guide.alpha;
 		// Every material here is non-delta, so NEE applies at every vertex of BNEEPT
 		// (TDirectLightEstimator::isNeeSamplable); a black Lambertian surface can gain nothing
 		// from it, so its shadow ray is skipped (its contribution would be exactly zero).
-		const bool black_matte = KIND == kShadeMatte &&
+		const bool black_matte = kMatte &&
 		                         ((mat.cr == 0.0f && mat.cg == 0.0f && mat.cb == 0.0f) || absorber);
 		const bool nee_samplable = !bvpt;
 		const bool use_nee = nee_samplable && s.num_emitters > 0 && !black_matte;
@@ -1141,7 +1160,7 @@ shade_kernel(ShadeArgs a)
 						// the direction-sampling technique at a guided vertex is the one-sample mixture
 						pdf_bsdf = alpha * guide_pdf(graw, l) + (1.0f - alpha) * pdf_bsdf;
 					}
-					if(GUIDED && guided && a.guide.train_cap)
+					if(guided && a.guide.train_cap)
 					{
 						// The light sample is a direction with known incident radiance and density:
 						// an importance-weighted sample of the incident-light distribution the network
@@ -1353,6 +1372,10 @@ void launch_shade(const ShadeArgs& sa, uint32_t kinds, int grid, cudaStream_t st
 	if(kinds & (1u << kShadeDielectric))
 	{
 		shade_kernel<GUIDED, MULTI, kShadeDielectric><<<grid, kShadeBlock, 0, st>>>(sa);
+	}
+	if constexpr(GUIDED)
+	{
+		shade_kernel<GUIDED, MULTI, kShadeGuided><<<grid, kShadeBlock, 0, st>>>(sa);
 	}
 	PG_CUDA_CHECK(cudaGetLastError());
 }
@@ -1794,7 +1817,6 @@ void RenderScene::ensure_guiding(uint32_t capacity)
 		}
 		m_st[0].resize(capacity);
 		m_st[1].resize(capacity);
-		m_gmap.resize(capacity);
 		m_gfeat.resize(static_cast<std::size_t>(capacity) * 8);
 		m_graw.resize(static_cast<std::size_t>(capacity) * guide::kMixFloats);
 		m_guide_capacity = capacity;
@@ -2596,7 +2618,6 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 			views[0].sqs[0].t = m_st[0].get();
 			views[0].sqs[1].t = m_st[1].get();
 		}
-		gargs.map = m_gmap.get();
 		gargs.feat = m_gfeat.get();
 		gargs.raw = m_graw.get();
 		gargs.train_feat = m_tfeat.get();
@@ -2706,7 +2727,8 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 		if(guided)
 		{
 			// network inputs of this iteration's guidable vertices, then the tensor-core forward pass
-			guide_query_kernel<<<grid, kShadeBlock, 0, st>>>(m_dev, d_counters, cur, w.hits.get(), gargs_b, guide_depth);
+			guide_query_kernel<<<grid, kShadeBlock, 0, st>>>(m_dev, d_counters, cur, w.hits.get(), gargs_b,
+			                                              w.order.get(), m_order_list);
 			PG_CUDA_CHECK(cudaGetLastError());
 			guide::launch_forward(m_gimage.get(), m_gfeat.get(), wave_capacity, nullptr, nullptr, m_gerr.get(), st,
 			                      &d_counters->n_guided, m_graw.get());
@@ -2955,7 +2977,8 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 			PG_CUDA_CHECK(cudaStreamSynchronize(st));
 			if(timing)
 			{
-				// event pairs: prepare, regen, extend, guide inference, shade, shadow, guide training
+				// event pairs: prepare (empty), begin, trace and classify, guide inference, shade and refine,
+				// shadow (empty), guide training
 				static const int slot[7] = {0, 1, 2, 5, 3, 4, 6};
 				for(int k = 0; k < 7; ++k)
 				{
@@ -2994,11 +3017,11 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 	m_last_iterations = iterations;
 	{
 		// begin, trace + classify, shade per material kind (+ refine in the iterative
-		// mode); guide query + forward; training: weight sums (and clamp), forward, backward, Adam,
+		// mode); guide query + forward + guided vertices' shading; training: weight sums (and clamp), forward, backward, Adam,
 		// step, loss
 		const unsigned long long per_iteration = 3ull + (classify ? 1ull : 0ull) + ((kinds >> kShadeConductor) & 1u) + ((kinds >> kShadeDielectric) & 1u) +
 		                                         (params.refine_mode == PG_REFINE_ITERATIVE ? 1ull : 0ull) +
-		                                         (guided ? 2ull : 0ull);
+		                                         (guided ? 3ull : 0ull);
 		const unsigned long long per_step = training ? (m_guide_params.clamp > 0.0f ? 8ull : 6ull) : 0ull;
 		// + the end of every period (graph mode), one training step per training period, and the film's
 		// box-weight or splat launch

@@ -75,8 +75,8 @@ enum RenderMode : uint32_t
 	PG_RENDER_COUNT = 2,    // plain launches, traversal kernels count nodes and triangles
 };
 
-// Progress of a render while it runs (graph mode). At every batch boundary -- the scene's stream
-// idle, every kernel of the batch complete, so the film holds exactly what finished paths put
+// Progress of a render while it runs (graph mode). At every progress point -- the loop on the device
+// ended for it and the scene's stream is idle, so the film holds exactly what finished paths put
 // there -- the film's estimate over the samples finished so far is developed into preview_rgb
 // (device memory, [h][w][3] float32, RGB / W with the box film's W counting finished samples
 // only) while `mutex` is held, and then `published` is called with the paths finished so far and
@@ -185,10 +185,10 @@ struct DeviceScene
 };
 
 // Shading classes of a closest-hit result. classify_kernel lists the queue slots of each class, and
-// each shading kernel takes the classes of its material kind: the matte kernel the first four (a
-// guided vertex also evaluates and samples the learned mixture: in a class of its own it fills whole
-// warps instead of making every matte warp wait on its guided lanes), the conductor and the
-// dielectric kernel one each. Each class has kClassLists lists, one per residue of the block index,
+// each shading kernel takes the classes of its kind: the matte kernel the first three, the others one
+// each (a guided vertex also evaluates and samples the learned mixture: in a class of its own it fills
+// whole warps instead of making every matte warp wait on its guided lanes; item w of that class has row
+// w of the network's inputs and outputs). Each class has kClassLists lists, one per residue of the block index,
 // so that the list counters' atomics spread over kOrderLists addresses instead of queuing on six.
 enum ShadeClass : uint32_t
 {
@@ -318,7 +318,6 @@ struct BatchView
 // Device view of the guiding buffers for one render iteration.
 struct GuideArgs
 {
-	uint32_t*       map = nullptr;        // queue entry -> network row, 0xFFFFFFFF = not guided
 	float*          feat = nullptr;       // [capacity][8] network input rows
 	const float*    raw = nullptr;        // [capacity][48] decoded mixtures (guide::kMixFloats per row)
 	float*          train_feat = nullptr; // [batch][8]: features 0-6, |cos| / pdf
@@ -373,11 +372,12 @@ public:
 	unsigned long long last_rays() const { return m_last_rays; }
 	unsigned long long last_shadow_rays() const { return m_last_shadow; }
 	unsigned long long last_iterations() const { return m_last_iterations; }
-	// Kernels launched by the last render (every iteration's launches, empty trailing iterations
-	// of the last graph batch included, and the per-render film launch).
+	// Kernels launched by the last render (every iteration's launches, the loop's own end kernels
+	// and the per-render film launch).
 	unsigned long long last_launches() const { return m_last_launches; }
-	// Per-kernel device milliseconds of the last timing-mode render: prepare, regen, extend,
-	// shade, shadow, guiding inference (query + network), guiding training.
+	// Per-kernel device milliseconds of the last timing-mode render: prepare (0: part of the next),
+	// regen (begin_kernel), extend (trace and classify), shade (and refine), shadow (0: traced by the
+	// next extend), guiding inference (query + network), guiding training.
 	const double* last_kernel_ms() const { return m_kernel_ms; }
 	// Nodes / triangles visited by closest-hit and any-hit queries in the last counting render.
 	const unsigned long long* last_counts() const { return m_last_counts; }
@@ -498,7 +498,6 @@ private:
 	float m_bound_lo[3] = {0, 0, 0}, m_bound_rcp[3] = {1, 1, 1};
 	DeviceBuffer<float4>   m_gf0[2], m_gf1[2];
 	DeviceBuffer<float4>   m_st[2];
-	DeviceBuffer<uint32_t> m_gmap;
 	DeviceBuffer<float>    m_gfeat, m_graw;
 	DeviceBuffer<float>    m_tfeat, m_traw;
 	DeviceBuffer<float4>   m_tdirw;

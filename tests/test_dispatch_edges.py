@@ -163,3 +163,25 @@ def test_two_wavefronts_give_one_wavefronts_film(gpu_lib, sample_filter, width, 
             rays.append((r["rays"], r["shadow_rays"]))
     assert rays[0] == rays[1]
     np.testing.assert_allclose(films[0], films[1], rtol=1e-11, atol=1e-11 * np.abs(films[1]).max())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("depth", [1, 0])
+@pytest.mark.parametrize("width,height,spp", [(1, 1, 1), (33, 31, 1), (45, 23, 3)])
+def test_guided_vertices_do_not_depend_on_their_row(gpu_lib, width, height, spp, depth):
+    """A guided vertex' row of the network is its place in the lists of its class: pools of 1,024 paths,
+    whose queues mix vertices of several bounces, against one that holds all paths; the network is frozen."""
+    import photon_gpu
+
+    scene = scenes.cornell_glossy(width, height, spp, 8)
+    films, guided = [], []
+    for capacity in (1024, 1 << 20):
+        with photon_gpu.RenderScene(scene) as rs:
+            rs.set_launch(capacity=capacity)
+            rs.set_guiding(True, False)
+            rs.set_guiding_depth(depth)
+            rs.render(spp, max_bounces=8, seed=23)
+            films.append(rs.film()[1])
+            guided.append(rs.guide_info()["guided_vertices"])
+    assert guided[0] == guided[1]
+    np.testing.assert_allclose(films[0], films[1], rtol=1e-11, atol=1e-11 * np.abs(films[1]).max())
