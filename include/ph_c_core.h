@@ -133,12 +133,13 @@ extern PH_API void phGpuClearFilm(PhUInt64 engineId);
 extern PH_API void phGpuGetRenderInfo(PhUInt64 engineId, PhFloat64* out_deviceMs, PhUInt64* out_paths,
                                       PhUInt64* out_rays, PhUInt64* out_shadowRays, PhFloat64* out_updateSeconds);
 
-/* Kernel launches of the last phRender (five per wavefront iteration). */
+/* Kernel launches of the last phRender (three to nine per wavefront iteration). */
 extern PH_API PhUInt64 phGpuGetLaunchCount(PhUInt64 engineId);
 /* Profiling render of `samplesPerPixel` samples into a scratch film (the engine's own image is
  * untouched). mode 1: plain launches with CUDA events around every kernel; mode 2: traversal
  * kernels count visited BVH nodes and tested triangles. out_stats (PhFloat64 [14]):
  *   [0..4] device ms of prepare, regen, extend (closest hit), shade, shadow (any hit) -- mode 1
+ *          (prepare and shadow are 0: their work is part of regen and extend)
  *   [5] total device ms, [6] paths, [7] closest-hit rays, [8] shadow rays, [9] iterations,
  *   [10] nodes visited by closest-hit rays, [11] triangles tested by them,
  *   [12] nodes visited by shadow rays, [13] triangles tested by them -- mode 2 */

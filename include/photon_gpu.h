@@ -207,7 +207,9 @@ PGPU_API int pgpu_scene_set_filter(uint64_t id, uint32_t filter);
  * phGpuSetDomePdf in ph_c_core.h. */
 PGPU_API int pgpu_scene_set_dome_pdf(uint64_t id, uint32_t mode);
 /* A render into a scratch film with every kernel bracketed by CUDA events: per-kernel device
- * milliseconds (prepare, regen, extend, shade, shadow, guide inference, guide training). */
+ * milliseconds (prepare, regen, extend, shade, shadow, guide inference, guide training). The names are
+ * older than the kernels: regen holds everything before the traversal and prepare is 0; the traversal
+ * serves both queues, so extend holds all of it and shadow is 0. */
 PGPU_API int pgpu_scene_profile(uint64_t id, uint32_t spp, uint32_t max_bounces, uint32_t estimator,
                        uint64_t seed, double* out_kernel_ms);
 PGPU_API int pgpu_scene_clear(uint64_t id);
@@ -274,8 +276,7 @@ PGPU_API int pgpu_scene_autotune(uint64_t id, uint32_t spp, uint32_t max_bounces
  * lanes), blocks per SM (1..64), leaf triangles (1..3; a different value rebuilds the BVH). */
 PGPU_API int pgpu_scene_set_launch(uint64_t id, const uint32_t* config);
 PGPU_API int pgpu_scene_get_launch(uint64_t id, uint32_t* out_config);
-/* Kernels the scene's last render launched (all iterations, including the empty ones that end the
- * last CUDA-graph batch). */
+/* Kernels the scene's last render launched (all iterations of all its wavefronts, and the film's). */
 PGPU_API int pgpu_scene_launches(uint64_t id, uint64_t* out_launches);
 /* A render into a scratch film whose traversal kernels count their work: out_counts uint64 [7] =
  * closest-hit rays, shadow rays, BVH nodes and triangles visited by closest-hit queries, the same
