@@ -322,7 +322,8 @@ backward_kernel(const float* __restrict__ params, const float* __restrict__ feat
 // are loaded while a round's MMAs run, and the input layer's two halves go through one round. The
 // CTAs' 3.8 M atomics on 29,480 addresses, four bytes each with every lane on a line of its own, had
 // been part of the 145 us that the kernel took at one thread per sample. 32 steps of 16,384 samples through
-// pgpu_guide_train went from 4.87 to 2.30 ms with this kernel and the fused Adam step.
+// pgpu_guide_train went from 4.87 to 2.30 ms with this kernel and the fused Adam step, and to 2.36 ms with
+// every bin of the input layer encoded by its own exponential.
 
 namespace tcb
 {
@@ -688,28 +689,19 @@ backward_tc_kernel(const float* __restrict__ params, const float* __restrict__ f
 			break;
 		}
 
-		// ---- layer 0: dW_0 of its 224 one-blob inputs, encoded as the forward pass encodes them; part 0
+		// ---- layer 0: dW_0 of its 224 one-blob inputs, each bin by its own exponential (the forward pass's
+		//      recurrence over a chunk of bins loses those of a chunk whose first one underflows); part 0
 		//      inputs 0, 2, 4 and 6, part 1 the others (unrolled so that f7 stays in registers)
 		#pragma unroll
 		for(int i = 0; i < kInputs; ++i)
 		{
 			if((i & 1) == static_cast<int>(part))
 			{
-				const float s32 = f7[i] * static_cast<float>(kBins) - 0.5f;
-				#pragma unroll
-				for(int c = 0; c < kBins / 8; ++c)
+				#pragma unroll 8
+				for(int b = 0; b < kBins; ++b)
 				{
-					const float z0 = s32 - static_cast<float>(c * 8);
-					float e = __expf(-0.5f * z0 * z0);
-					float ratio = __expf(z0 - 0.5f);
-					#pragma unroll
-					for(int j = 0; j < 8; ++j)
-					{
-						const uint32_t k = static_cast<uint32_t>(i * kBins + c * 8 + j);
-						st_bf16(k < 128u ? xt : xt + kXtBytes, core_offset_lbo(k & 127u, r, kLboXT), valid ? e : 0.0f);
-						e *= ratio;
-						ratio *= 0.36787944117144233f;   // e^-1
-					}
+					const uint32_t k = static_cast<uint32_t>(i * kBins + b);
+					st_bf16(i < 4 ? xt : xt + kXtBytes, core_offset_lbo(k & 127u, r, kLboXT), valid ? one_blob(f7[i], b) : 0.0f);
 				}
 			}
 		}
