@@ -52,9 +52,10 @@ void launch_gradients(const float* d_params, const unsigned char* d_image, const
 
 // One Adam step (beta 0.9 / 0.999, eps 1e-8) on the FP32 parameters with the gradient that
 // launch_gradients left in d_partials for the same n and d_n; d_image receives the new weights. The
-// step number t is *d_step + 1, and *d_step is incremented afterwards (graph-safe).
+// step number t is *d_step + 1, and *d_step is incremented afterwards (graph-safe). With *d_error set
+// (a network kernel gave up: its gradient is incomplete) the step is left out and nothing changes.
 void launch_adam(float* d_params, const float* d_partials, uint32_t n, const uint32_t* d_n, float* d_m, float* d_v,
-                 uint32_t* d_step, unsigned char* d_image, float lr, cudaStream_t s);
+                 uint32_t* d_step, unsigned char* d_image, float lr, const uint32_t* d_error, cudaStream_t s);
 
 }// end namespace guide
 }// end namespace pg

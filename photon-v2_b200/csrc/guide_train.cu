@@ -22,6 +22,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <cstring>
 #include <vector>
 
 namespace pg
@@ -791,11 +792,14 @@ __device__ __forceinline__ float sum_partials(const float* __restrict__ partials
 	return s;
 }
 
+// A CTA of the backward kernel that gave up waiting on its tensor cores left no row in `partials`: with
+// the error word set, the rows are not summed and the state stays as it was before the step.
+
 __global__ void reduce_partials_kernel(const float* __restrict__ partials, uint32_t n_max, const uint32_t* __restrict__ d_n,
-                                       uint32_t grid, float* __restrict__ grads)
+                                       uint32_t grid, const uint32_t* __restrict__ error, float* __restrict__ grads)
 {
 	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-	if(i < kNumParams)
+	if(i < kNumParams && *error == 0u)
 	{
 		grads[i] += sum_partials(partials, partial_rows(n_max, d_n, grid), i);
 	}
@@ -806,10 +810,11 @@ __global__ void reduce_partials_kernel(const float* __restrict__ partials, uint3
 __global__ void adam_kernel(float* __restrict__ params, const float* __restrict__ partials, uint32_t n_max,
                             const uint32_t* __restrict__ d_n, uint32_t grid, float* __restrict__ m,
                             float* __restrict__ v, float lr, float beta1, float beta2, float eps,
-                            const uint32_t* __restrict__ step, unsigned char* __restrict__ image)
+                            const uint32_t* __restrict__ step, const uint32_t* __restrict__ error,
+                            unsigned char* __restrict__ image)
 {
 	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-	if(i >= kNumParams)
+	if(i >= kNumParams || *error != 0u)
 	{
 		return;
 	}
@@ -826,9 +831,9 @@ __global__ void adam_kernel(float* __restrict__ params, const float* __restrict_
 	store_image(image, i, w);
 }
 
-__global__ void step_kernel(uint32_t* step)
+__global__ void step_kernel(uint32_t* step, const uint32_t* error)
 {
-	++*step;
+	*step += *error == 0u ? 1u : 0u;
 }
 
 uint32_t backward_grid(uint32_t n)
@@ -875,7 +880,7 @@ void launch_gradients(const float* d_params, const unsigned char* d_image, const
 		PG_CUDA_CHECK(cudaGetLastError());
 		if(d_grads)
 		{
-			reduce_partials_kernel<<<(kNumParams + 127) / 128, 128, 0, s>>>(d_partials, n, d_n, grid, d_grads);
+			reduce_partials_kernel<<<(kNumParams + 127) / 128, 128, 0, s>>>(d_partials, n, d_n, grid, d_error, d_grads);
 			PG_CUDA_CHECK(cudaGetLastError());
 		}
 		return;
@@ -888,12 +893,12 @@ void launch_gradients(const float* d_params, const unsigned char* d_image, const
 }
 
 void launch_adam(float* d_params, const float* d_partials, uint32_t n, const uint32_t* d_n, float* d_m, float* d_v,
-                 uint32_t* d_step, unsigned char* d_image, float lr, cudaStream_t s)
+                 uint32_t* d_step, unsigned char* d_image, float lr, const uint32_t* d_error, cudaStream_t s)
 {
 	adam_kernel<<<(kNumParams + 127) / 128, 128, 0, s>>>(d_params, d_partials, n, d_n, backward_grid(n), d_m, d_v, lr, 0.9f,
-	                                                     0.999f, 1e-8f, d_step, d_image);
+	                                                     0.999f, 1e-8f, d_step, d_error, d_image);
 	PG_CUDA_CHECK(cudaGetLastError());
-	step_kernel<<<1, 1, 0, s>>>(d_step);
+	step_kernel<<<1, 1, 0, s>>>(d_step, d_error);
 	PG_CUDA_CHECK(cudaGetLastError());
 }
 
@@ -994,11 +999,14 @@ int pgpu_guide_train(float* params, const float* features, const float* dirs, co
 			                        d_dirw.get() + first, count, d_raw.get(), d_acts.get(), d_partials.get(), nullptr,
 			                        d_scalars.get() + 2 * step, d_scalars.get() + 2 * step + 1, d_err.get(), s);
 			guide::launch_adam(d_params.get(), d_partials.get(), count, nullptr, d_m.get(), d_v.get(), d_step.get(),
-			                   d_image.get(), lr, s);
+			                   d_image.get(), lr, d_err.get(), s);
 		}
 		std::vector<float> scalars(2 * static_cast<std::size_t>(steps));
 		uint32_t err = 0;
-		PG_CUDA_CHECK(cudaMemcpyAsync(params, d_params.get(), d_params.bytes(), cudaMemcpyDeviceToHost, s));
+		// (through the stage: the caller's parameters stay as they are if a step failed)
+		static_assert(guide::kNumParams * sizeof(float) <= kPinnedStage, "page-locked stage");
+		const unsigned char* const trained = pinned_stage();
+		PG_CUDA_CHECK(cudaMemcpyAsync(pinned_stage(), d_params.get(), d_params.bytes(), cudaMemcpyDeviceToHost, s));
 		PG_CUDA_CHECK(cudaMemcpyAsync(scalars.data(), d_scalars.get(), d_scalars.bytes(), cudaMemcpyDeviceToHost, s));
 		PG_CUDA_CHECK(cudaMemcpyAsync(&err, d_err.get(), sizeof(err), cudaMemcpyDeviceToHost, s));
 		PG_CUDA_CHECK(cudaStreamSynchronize(s));
@@ -1006,6 +1014,7 @@ int pgpu_guide_train(float* params, const float* features, const float* dirs, co
 		{
 			throw Error(PG_ERR_CUDA, "guiding network: tensor-core wait timed out");
 		}
+		std::memcpy(params, trained, d_params.bytes());
 		if(out_losses)
 		{
 			for(uint32_t i = 0; i < steps; ++i)

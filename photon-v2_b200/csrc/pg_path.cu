@@ -2782,7 +2782,7 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 			                        m_gscalars.get(), m_gscalars.get() + 1, m_gerr.get(), st, &d_counters->n_train,
 			                        m_guide_params.clamp);
 			guide::launch_adam(m_gparams.get(), m_gpartials.get(), train_cap, &d_counters->n_train, m_gm.get(), m_gv.get(),
-			                   m_gstep.get(), m_gimage.get(), m_guide_params.lr, st);
+			                   m_gstep.get(), m_gimage.get(), m_guide_params.lr, m_gerr.get(), st);
 			guide_loss_kernel<<<1, 1, 0, st>>>(m_gscalars.get(), &d_counters->n_train);
 			PG_CUDA_CHECK(cudaGetLastError());
 		}
