@@ -623,15 +623,15 @@ __host__ __device__ inline bool render_done(const RenderCounters& c)
 // The end of a period of iterations: whether the graph's loop runs another one. It ends when every
 // path has finished, on an error (an iteration with nothing in its queues before that is one), at a
 // progress point (pause_at, for renders that publish previews; the points' distance doubles up to
-// 128 iterations) and, as a backstop, after kMaxIterations.
+// max_pause_step iterations) and, as a backstop, after kMaxIterations.
 constexpr uint32_t kMaxIterations = 1u << 25;
 
-__global__ void end_kernel(RenderCounters* c, cudaGraphConditionalHandle loop)
+__global__ void end_kernel(RenderCounters* c, uint32_t max_pause_step, cudaGraphConditionalHandle loop)
 {
 	const bool pause = c->iterations >= c->pause_at;
 	if(pause)
 	{
-		c->pause_step = min(c->pause_step * 2u, 128u);
+		c->pause_step = min(c->pause_step * 2u, max_pause_step);
 		c->pause_at = c->iterations + c->pause_step;
 	}
 	const bool done = render_done(*c);
@@ -2372,8 +2372,9 @@ float RenderScene::render_batch(const std::vector<const RenderScene*>& scenes, c
 // split into passes of whole samples per pixel.
 constexpr unsigned long long kMaxFilteredPassPaths = 1ull << 27;
 constexpr unsigned long long kMaxBoxPassPaths = 1ull << 31;
-// Iterations up to the first progress point of a render that publishes previews.
-constexpr uint32_t kFirstPause = 16;
+// Periods of iterations up to the first progress point of a render that publishes previews, and at most
+// between two: a short render of five periods shows one preview, a long one is not held up.
+constexpr uint32_t kFirstPausePeriods = 4, kMaxPausePeriods = 64;
 
 float RenderScene::render(const RenderParams& params, double* film_sums)
 {
@@ -2501,6 +2502,8 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 	const int grid = sms * static_cast<int>(lc.blocks_per_sm);   // grid-stride kernels: 128-thread blocks
 	const int refill = static_cast<int>(lc.refill);
 	const bool guided = m_guide_params.enabled && params.estimator == PG_EST_BNEEPT;   // (BNEEPT only)
+	const bool training = guided && m_guide_params.train;
+	const int period = training ? kTrainPeriod : 2;   // iterations (the two path buffers; training: see gargs_of)
 
 	// Two wavefronts, each with half of the paths and of the pool, run side by side on streams of their
 	// own: a traversal launch ends with a tail of its longest rays (a fifth of its time on the bench
@@ -2587,8 +2590,8 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 		*x.host = RenderCounters{};
 		x.host->next_path = x.first;
 		x.host->total_paths = x.end;
-		x.host->pause_at = params.progress ? kFirstPause : 0xFFFFFFFFu;
-		x.host->pause_step = kFirstPause;
+		x.host->pause_step = kFirstPausePeriods * static_cast<uint32_t>(period);
+		x.host->pause_at = params.progress ? x.host->pause_step : 0xFFFFFFFFu;
 		x.wave->host_state->consts = RenderConsts{params.seed, first_global};
 		PG_CUDA_CHECK(cudaMemcpyAsync(x.wave->state.get(), x.wave->host_state, kStateHead, cudaMemcpyHostToDevice, st));
 	}
@@ -2600,7 +2603,6 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 	const uint32_t guide_depth = !guided ? 0u
 	                             : (m_guide_params.depth == 0u || m_guide_params.depth > max_bounces ? max_bounces
 	                                                                                                : m_guide_params.depth);
-	const bool training = guided && m_guide_params.train;
 	GuideArgs gargs;
 	uint32_t train_cap = 0;
 	if(guided)
@@ -2660,7 +2662,6 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 	//   q = P-1      open samples collect the emission found; the iteration ends with one Adam step.
 	// The trace of q = 2 ... P-1 resolves the NEE of q = 1 ... P-2, so every credit lands before
 	// the step. Without training the period is two iterations (the two path buffers).
-	const int period = training ? kTrainPeriod : 2;
 	GuideArgs gargs_of[kTrainPeriod];
 	for(int q = 0; q < kTrainPeriod; ++q)
 	{
@@ -2899,7 +2900,7 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 					{
 						iteration(x, q, nullptr);
 					}
-					end_kernel<<<1, 1, 0, x.wave->stream>>>(x.counters[1], loop);
+					end_kernel<<<1, 1, 0, x.wave->stream>>>(x.counters[1], kMaxPausePeriods * static_cast<uint32_t>(period), loop);
 					PG_CUDA_CHECK(cudaGetLastError());
 				});
 				x.wave->exec_key = key;
