@@ -513,15 +513,14 @@ __device__ __forceinline__ uint32_t alloc_slot(uint32_t* counter)
 // its scene in the top bits of its meta word.
 template<bool MULTI>
 __global__ void __launch_bounds__(kShadeBlock)
-begin_kernel(const RenderCounters* __restrict__ prev, RenderCounters* __restrict__ c, uint32_t capacity,
-             uint32_t period_pos, uint32_t record_budget, Camera cam_single, FilmView film_single,
+begin_kernel(const RenderCounters* __restrict__ prev, RenderCounters* __restrict__ c, uint32_t period_pos, uint32_t record_budget, Camera cam_single, FilmView film_single,
              const RenderConsts* __restrict__ k,
              PathBuffers cur, BatchView batch)
 {
 	const uint32_t active = prev->n_next;
 	const unsigned long long base = prev->next_path;
 	const unsigned long long remaining = prev->total_paths - base;
-	const unsigned long long room = static_cast<unsigned long long>(capacity - active);
+	const unsigned long long room = static_cast<unsigned long long>(prev->capacity - active);
 	const uint32_t n_new = static_cast<uint32_t>(remaining < room ? remaining : room);
 	const uint32_t total = active + n_new;
 	if(blockIdx.x == 0)
@@ -539,6 +538,7 @@ begin_kernel(const RenderCounters* __restrict__ prev, RenderCounters* __restrict
 			c->n_shadow_prev = prev->n_shadow;
 			c->next_path = base + n_new;
 			c->total_paths = prev->total_paths;
+			c->capacity = prev->capacity;
 			c->rays_traced = prev->rays_traced + total;
 			c->shadow_rays = prev->shadow_rays + prev->n_shadow;   // traced in this iteration
 			c->nodes_closest = prev->nodes_closest;
@@ -782,7 +782,6 @@ struct ShadeArgs
 	RenderCounters* counters;
 	FilmView      film;
 	const RenderConsts* consts;
-	uint32_t      max_bounces;
 	uint32_t      estimator;
 	uint32_t      width_height;
 	GuideArgs     guide;
@@ -1028,7 +1027,7 @@ shade_kernel(ShadeArgs a)
 		}
 
 		// ---- does the path continue past this vertex?
-		if((meta & kMetaStopAfter) || bounce >= a.max_bounces)
+		if((meta & kMetaStopAfter) || bounce >= consts.max_bounces)
 		{
 			splat(film, pixel, p, radiance);
 			continue;
@@ -1715,9 +1714,9 @@ RenderScene::~RenderScene()
 {
 	for(Wave& w : m_waves)
 	{
-		if(w.exec)
+		for(const LoopGraph& g : w.graphs)
 		{
-			cudaGraphExecDestroy(w.exec);
+			cudaGraphExecDestroy(g.exec);
 		}
 		if(w.stream)
 		{
@@ -1740,67 +1739,79 @@ RenderScene::~RenderScene()
 
 void RenderScene::ensure_capacity(uint32_t waves, uint32_t capacity, uint32_t grid)
 {
-	if(waves <= m_pool_waves && capacity <= m_capacity && grid == m_order_grid)
+	if(capacity <= m_layouts[waves - 1u].capacity && grid == m_order_grid)
 	{
 		return;
 	}
 	++m_buffer_generation;
-	// the slots the blocks of one residue visit in classify_kernel's grid-stride loop
-	const uint32_t rounds = (capacity + grid * kShadeBlock - 1u) / (grid * kShadeBlock);
-	m_order_list = (grid + kClassLists - 1u) / kClassLists * rounds * kShadeBlock;
+	uint32_t wanted[kMaxWaves];
+	for(uint32_t n = 1; n <= kMaxWaves; ++n)
+	{
+		wanted[n - 1u] = std::max(m_layouts[n - 1u].capacity, n == waves ? capacity : 0u);
+	}
 	// One allocation for the whole pool (0.8 GB at 2^21 slots): about thirty of them, one per array,
 	// took most of a new scene's first render of a small image. Two rounds: sizes, then addresses.
 	std::size_t total = 0;
 	for(int round = 0; round < 2; ++round)
 	{
 		unsigned char* const base = round == 0 ? nullptr : m_pool.get();
-		std::size_t at = 0;
-		auto carve = [&](auto& span, std::size_t n)
+		for(uint32_t n = 1; n <= kMaxWaves; ++n)
 		{
-			using T = std::remove_pointer_t<decltype(span.get())>;
+			const uint32_t slots = wanted[n - 1u];
+			PoolLayout& layout = m_layouts[n - 1u];
+			// the slots the blocks of one residue visit in classify_kernel's grid-stride loop
+			const uint32_t rounds = (slots + grid * kShadeBlock - 1u) / (grid * kShadeBlock);
+			const uint32_t order_list = (grid + kClassLists - 1u) / kClassLists * rounds * kShadeBlock;
+			std::size_t at = 0;
+			auto carve = [&](auto& span, std::size_t count)
+			{
+				using T = std::remove_pointer_t<decltype(span.get())>;
+				if(base)
+				{
+					span.set(base + at, count);
+				}
+				at += (count * sizeof(T) + 255u) / 256u * 256u;
+			};
+			for(uint32_t k = 0; k < (slots ? n : 0u); ++k)
+			{
+				WaveBuffers& w = layout.buffers[k];
+				for(int b = 0; b < 2; ++b)
+				{
+					carve(w.path[b], slots);
+					carve(w.meta[b], slots);
+					carve(w.thr[b], slots);
+					carve(w.rad[b], slots);
+					carve(w.prev[b], slots);
+					carve(w.ro[b], slots);
+					carve(w.rd[b], slots);
+					carve(w.so[b], slots);
+					carve(w.sd[b], slots);
+					carve(w.sc[b], slots);
+					carve(w.sr[b], slots);
+					carve(w.sid[b], slots);
+				}
+				carve(w.hits, slots);
+				carve(w.req_single, slots);
+				carve(w.req_mutual, slots);
+				carve(w.order, static_cast<std::size_t>(kOrderLists) * order_list);
+			}
+			total = std::max(total, at);
 			if(base)
 			{
-				span.set(base + at, n);
+				layout.capacity = slots;
+				layout.order_list = order_list;
 			}
-			at += (n * sizeof(T) + 255u) / 256u * 256u;
-		};
-		for(uint32_t k = 0; k < waves; ++k)
-		{
-			Wave& w = m_waves[k];
-			for(int b = 0; b < 2; ++b)
-			{
-				carve(w.path[b], capacity);
-				carve(w.meta[b], capacity);
-				carve(w.thr[b], capacity);
-				carve(w.rad[b], capacity);
-				carve(w.prev[b], capacity);
-				carve(w.ro[b], capacity);
-				carve(w.rd[b], capacity);
-				carve(w.so[b], capacity);
-				carve(w.sd[b], capacity);
-				carve(w.sc[b], capacity);
-				carve(w.sr[b], capacity);
-				carve(w.sid[b], capacity);
-			}
-			carve(w.hits, capacity);
-			carve(w.req_single, capacity);
-			carve(w.req_mutual, capacity);
-			carve(w.order, static_cast<std::size_t>(kOrderLists) * m_order_list);
 		}
-		if(round == 0)
+		if(round == 0 && total > m_pool.size())
 		{
-			total = at;
-			if(total > m_pool.size())
+			for(PoolLayout& layout : m_layouts)
 			{
-				m_capacity = 0;      // the old pool goes first
-				m_pool_waves = 0;
-				m_pool.release();
-				m_pool.resize(total);
+				layout.capacity = 0;   // the old pool goes first
 			}
+			m_pool.release();
+			m_pool.resize(total);
 		}
 	}
-	m_pool_waves = waves;
-	m_capacity = capacity;
 	m_order_grid = grid;
 }
 
@@ -2375,6 +2386,8 @@ constexpr unsigned long long kMaxBoxPassPaths = 1ull << 31;
 // Periods of iterations up to the first progress point of a render that publishes previews, and at most
 // between two: a short render of five periods shows one preview, a long one is not held up.
 constexpr uint32_t kFirstPausePeriods = 4, kMaxPausePeriods = 64;
+// Loop graphs kept per wave: what a program alternates (plain and guided, two films or estimators) stays.
+constexpr std::size_t kKeptGraphs = 4;
 
 float RenderScene::render(const RenderParams& params, double* film_sums)
 {
@@ -2426,15 +2439,10 @@ uint64_t float_bits(float v)
 
 }// end anonymous namespace
 
-// Captures `launches` (on the wave's stream; given the loop's handle) as the body of a loop on the
-// device and instantiates it as the wave's graph.
-void RenderScene::build_loop_graph(Wave& wave, const std::function<void(cudaGraphConditionalHandle)>& launches)
+// Captures `launches` (on the stream; given the loop's handle) as the body of a loop on the device and
+// instantiates it.
+cudaGraphExec_t RenderScene::build_loop_graph(cudaStream_t stream, const std::function<void(cudaGraphConditionalHandle)>& launches)
 {
-	if(wave.exec)
-	{
-		PG_CUDA_CHECK(cudaGraphExecDestroy(wave.exec));
-		wave.exec = nullptr;
-	}
 	struct GraphHolder
 	{
 		cudaGraph_t g = nullptr;
@@ -2450,7 +2458,7 @@ void RenderScene::build_loop_graph(Wave& wave, const std::function<void(cudaGrap
 	node.conditional.size = 1;
 	cudaGraphNode_t added;
 	PG_CUDA_CHECK(cudaGraphAddNode(&added, holder.g, nullptr, 0, &node));
-	PG_CUDA_CHECK(cudaStreamBeginCaptureToGraph(wave.stream, node.conditional.phGraph_out[0], nullptr, nullptr, 0,
+	PG_CUDA_CHECK(cudaStreamBeginCaptureToGraph(stream, node.conditional.phGraph_out[0], nullptr, nullptr, 0,
 	                                            cudaStreamCaptureModeThreadLocal));
 	try
 	{
@@ -2459,13 +2467,15 @@ void RenderScene::build_loop_graph(Wave& wave, const std::function<void(cudaGrap
 	catch(...)
 	{
 		cudaGraph_t body;
-		cudaStreamEndCapture(wave.stream, &body);
+		cudaStreamEndCapture(stream, &body);
 		(void)cudaGetLastError();
 		throw;
 	}
 	cudaGraph_t body;
-	PG_CUDA_CHECK(cudaStreamEndCapture(wave.stream, &body));
-	PG_CUDA_CHECK(cudaGraphInstantiate(&wave.exec, holder.g, 0));
+	PG_CUDA_CHECK(cudaStreamEndCapture(stream, &body));
+	cudaGraphExec_t exec = nullptr;
+	PG_CUDA_CHECK(cudaGraphInstantiate(&exec, holder.g, 0));
+	return exec;
 }
 
 float RenderScene::render_pass(const RenderParams& params, double* film_sums, const std::vector<BatchScene>* batch)
@@ -2516,18 +2526,21 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 	const uint32_t waves = params.mode == PG_RENDER_GRAPH && !guided && total >= 2ull * capacity ? 2u : 1u;
 	const uint32_t wave_capacity = (capacity + waves - 1u) / waves;
 	ensure_capacity(waves, std::max<uint32_t>(wave_capacity, 1024u), static_cast<uint32_t>(grid));
+	const PoolLayout& layout = m_layouts[waves - 1u];
 
 	cudaStream_t const st = m_stream;
 	// each wave's buffers by iteration parity, counter sets and pinned counters
 	struct WaveView
 	{
 		Wave*           wave;
+		const WaveBuffers* pool;
 		PathBuffers     buf[2];
 		ShadowQueue     sqs[2];
 		RenderCounters* counters[2];
 		const RenderConsts* consts;
 		RenderCounters* host;
 		unsigned long long first, end;   // its paths
+		cudaGraphExec_t exec;
 		bool            done;
 	};
 	WaveView views[kMaxWaves];
@@ -2546,13 +2559,15 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 		WaveView& x = views[v];
 		x = WaveView{};
 		x.wave = &w;
+		const WaveBuffers& p = layout.buffers[v];
+		x.pool = &p;
 		for(int b = 0; b < 2; ++b)
 		{
-			x.buf[b] = PathBuffers{w.path[b].get(), w.meta[b].get(), w.thr[b].get(), w.rad[b].get(),
-			                       w.prev[b].get(), w.ro[b].get(), w.rd[b].get()};
-			x.sqs[b] = ShadowQueue{w.so[b].get(), w.sd[b].get(), w.sc[b].get()};
-			x.sqs[b].r = w.sr[b].get();
-			x.sqs[b].sid = multi ? w.sid[b].get() : nullptr;
+			x.buf[b] = PathBuffers{p.path[b].get(), p.meta[b].get(), p.thr[b].get(), p.rad[b].get(),
+			                       p.prev[b].get(), p.ro[b].get(), p.rd[b].get()};
+			x.sqs[b] = ShadowQueue{p.so[b].get(), p.sd[b].get(), p.sc[b].get()};
+			x.sqs[b].r = p.sr[b].get();
+			x.sqs[b].sid = multi ? p.sid[b].get() : nullptr;
 			x.counters[b] = &w.state.get()->counters[1 - b];   // the iteration before the first: set 0
 		}
 		x.consts = &w.state.get()->consts;
@@ -2581,6 +2596,8 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 		}
 		film.samples = m_samples.get();
 	}
+	// BVPTDL follows one BSDF-sampled bounce whatever the configured depth (BVPTDLEstimator.cpp:62-95)
+	const uint32_t max_bounces = params.estimator == PG_EST_BVPTDL ? 1u : params.max_bounces;
 	const uint64_t first_global = params.first_sample * wh;
 	// what changes from render to render goes through device memory, so that a scene's graph serves
 	// all its renders of one shape
@@ -2590,14 +2607,13 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 		*x.host = RenderCounters{};
 		x.host->next_path = x.first;
 		x.host->total_paths = x.end;
+		x.host->capacity = wave_capacity;
 		x.host->pause_step = kFirstPausePeriods * static_cast<uint32_t>(period);
 		x.host->pause_at = params.progress ? x.host->pause_step : 0xFFFFFFFFu;
-		x.wave->host_state->consts = RenderConsts{params.seed, first_global};
+		x.wave->host_state->consts = RenderConsts{params.seed, first_global, max_bounces};
 		PG_CUDA_CHECK(cudaMemcpyAsync(x.wave->state.get(), x.wave->host_state, kStateHead, cudaMemcpyHostToDevice, st));
 	}
 	const bool counting = params.mode == PG_RENDER_COUNT;
-	// BVPTDL follows one BSDF-sampled bounce whatever the configured depth (BVPTDLEstimator.cpp:62-95)
-	const uint32_t max_bounces = params.estimator == PG_EST_BVPTDL ? 1u : params.max_bounces;
 
 	// learned guiding: the vertices a guided render guides: those below this bounce (0: none)
 	const uint32_t guide_depth = !guided ? 0u
@@ -2607,7 +2623,7 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 	uint32_t train_cap = 0;
 	if(guided)
 	{
-		ensure_guiding(m_capacity);
+		ensure_guiding(layout.capacity);
 		train_cap = training ? std::max<uint32_t>(m_guide_params.batch, guide::kTile) : 0u;
 		for(int b = 0; b < 2; ++b)
 		{
@@ -2682,8 +2698,8 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 	auto iteration = [&](WaveView& x, int q, cudaEvent_t* ev)
 	{
 		const int b = q & 1;
-		Wave& w = *x.wave;
-		cudaStream_t const st = w.stream;
+		const WaveBuffers& w = *x.pool;
+		cudaStream_t const st = x.wave->stream;
 		const PathBuffers& cur = x.buf[b];
 		const PathBuffers& nxt = x.buf[1 - b];
 		RenderCounters* const d_counters = x.counters[b];
@@ -2693,12 +2709,12 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 		const uint32_t pos = training ? static_cast<uint32_t>(q) : 2u;
 		if(multi)
 		{
-			begin_kernel<true><<<grid, kShadeBlock, 0, st>>>(x.counters[1 - b], d_counters, wave_capacity, pos,
+			begin_kernel<true><<<grid, kShadeBlock, 0, st>>>(x.counters[1 - b], d_counters, pos,
 			                                                 train_cap / 4u * 3u, m_dev.cam, film, x.consts, cur, bview);
 		}
 		else
 		{
-			begin_kernel<false><<<grid, kShadeBlock, 0, st>>>(x.counters[1 - b], d_counters, wave_capacity, pos,
+			begin_kernel<false><<<grid, kShadeBlock, 0, st>>>(x.counters[1 - b], d_counters, pos,
 			                                                  train_cap / 4u * 3u, m_dev.cam, film, x.consts, cur, bview);
 		}
 		PG_CUDA_CHECK(cudaGetLastError());
@@ -2715,12 +2731,12 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 		else if(multi)
 		{
 			classify_kernel<true><<<grid, kShadeBlock, 0, st>>>(m_dev, d_counters, w.hits.get(), w.order.get(),
-			                                                    m_order_list, cur.meta, bview, 0u);
+			                                                    layout.order_list, cur.meta, bview, 0u);
 		}
 		else
 		{
 			classify_kernel<false><<<grid, kShadeBlock, 0, st>>>(m_dev, d_counters, w.hits.get(), w.order.get(),
-			                                                     m_order_list, cur.meta, bview, guide_depth);
+			                                                     layout.order_list, cur.meta, bview, guide_depth);
 		}
 		PG_CUDA_CHECK(cudaGetLastError());
 		if(ev) { PG_CUDA_CHECK(cudaEventRecord(ev[3], st)); }
@@ -2729,13 +2745,13 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 		{
 			// network inputs of this iteration's guidable vertices, then the tensor-core forward pass
 			guide_query_kernel<<<grid, kShadeBlock, 0, st>>>(m_dev, d_counters, cur, w.hits.get(), gargs_b,
-			                                              w.order.get(), m_order_list);
+			                                              w.order.get(), layout.order_list);
 			PG_CUDA_CHECK(cudaGetLastError());
 			guide::launch_forward(m_gimage.get(), m_gfeat.get(), wave_capacity, nullptr, nullptr, m_gerr.get(), st,
 			                      &d_counters->n_guided, m_graw.get());
 		}
 		if(ev) { PG_CUDA_CHECK(cudaEventRecord(ev[4], st)); }
-		ShadeArgs sa{m_dev, cur, nxt, w.hits.get(), sq, d_counters, film, x.consts, max_bounces, params.estimator,
+		ShadeArgs sa{m_dev, cur, nxt, w.hits.get(), sq, d_counters, film, x.consts, params.estimator,
 		             static_cast<uint32_t>(wh)};
 		sa.guide = gargs_b;
 		sa.refine.mode = params.refine_mode;
@@ -2743,7 +2759,7 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 		sa.refine.iters = static_cast<int>(params.refine_iters);
 		sa.refine_queue = queue_nee ? RefineQueue{w.req_single.get(), w.req_mutual.get()} : RefineQueue{};
 		sa.order = classify ? w.order.get() : nullptr;
-		sa.order_capacity = m_order_list;
+		sa.order_capacity = layout.order_list;
 		sa.batch = bview;
 		if(multi)
 		{
@@ -2874,16 +2890,29 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 		// training): the last kernel of a period decides whether another follows, so that no
 		// iteration runs after the last path and the host only waits. (Periods launched by the host
 		// in batches of 4, 8, ... ran up to 14 empty iterations on short renders: a 64 x 48 thumbnail
-		// took 24 iterations for its 9.) The graph is built again only when something its launches
-		// were given has changed.
+		// took 24 iterations for its 9.) Building a graph takes about 270 us, more than a thumbnail's whole
+		// render, so a wave keeps those of the last kinds of render, and what changes from call to
+		// call (samples, depth, seed, pool share) reaches the kernels through device memory.
+		if(m_graph_generation != m_buffer_generation)
+		{
+			for(Wave& w : m_waves)
+			{
+				for(const LoopGraph& g : w.graphs)
+				{
+					cudaGraphExecDestroy(g.exec);   // names buffers that are gone
+				}
+				w.graphs.clear();
+			}
+			m_graph_generation = m_buffer_generation;
+		}
 		std::vector<uint64_t> key = {static_cast<uint64_t>(period), waves, guided, training, multi, kinds, static_cast<uint64_t>(grid),
-		                             wave_capacity, static_cast<uint64_t>(refill), m_order_list, max_bounces, params.estimator, wh,
-		                             params.refine_mode, float_bits(params.refine_delta), params.refine_iters,
-		                             m_dev.env_map.exact, guide_depth, train_cap, bview.count, m_buffer_generation,
+		                             static_cast<uint64_t>(refill), params.estimator, wh, params.refine_mode,
+		                             float_bits(params.refine_delta), params.refine_iters, m_dev.env_map.exact, bview.count,
 		                             params.filter, queue_nee,
 		                             reinterpret_cast<uint64_t>(film.sums), reinterpret_cast<uint64_t>(film.samples)};
 		if(guided)
 		{
+			key.insert(key.end(), {wave_capacity, guide_depth, train_cap});
 			for(float v : {m_guide_params.alpha, m_guide_params.lr, m_guide_params.clamp})
 			{
 				key.push_back(float_bits(v));
@@ -2892,9 +2921,11 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 		for(uint32_t v = 0; v < waves; ++v)
 		{
 			WaveView& x = views[v];
-			if(!x.wave->exec || x.wave->exec_key != key)
+			std::vector<LoopGraph>& graphs = x.wave->graphs;
+			auto found = std::find_if(graphs.begin(), graphs.end(), [&](const LoopGraph& g) { return g.key == key; });
+			if(found == graphs.end())
 			{
-				build_loop_graph(*x.wave, [&](cudaGraphConditionalHandle loop)
+				const cudaGraphExec_t exec = build_loop_graph(x.wave->stream, [&](cudaGraphConditionalHandle loop)
 				{
 					for(int q = 0; q < period; ++q)
 					{
@@ -2903,8 +2934,15 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 					end_kernel<<<1, 1, 0, x.wave->stream>>>(x.counters[1], kMaxPausePeriods * static_cast<uint32_t>(period), loop);
 					PG_CUDA_CHECK(cudaGetLastError());
 				});
-				x.wave->exec_key = key;
+				if(graphs.size() == kKeptGraphs)
+				{
+					cudaGraphExecDestroy(graphs.back().exec);
+					graphs.pop_back();
+				}
+				found = graphs.insert(graphs.end(), LoopGraph{exec, key});
 			}
+			std::rotate(graphs.begin(), found, found + 1);
+			x.exec = graphs.front().exec;
 		}
 		// (should a call below throw, nothing of this render is left running on the other stream)
 		struct WaitForWaves
@@ -2933,7 +2971,7 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 				WaveView& x = views[v];
 				if(!x.done)
 				{
-					PG_CUDA_CHECK(cudaGraphLaunch(x.wave->exec, x.wave->stream));
+					PG_CUDA_CHECK(cudaGraphLaunch(x.exec, x.wave->stream));
 					PG_CUDA_CHECK(cudaMemcpyAsync(x.host, x.counters[1], kCountersHead, cudaMemcpyDeviceToHost, x.wave->stream));
 				}
 			}

@@ -213,6 +213,7 @@ struct alignas(128) RenderCounters
 {
 	uint32_t n_total;       // paths in the queue: the previous iteration's n_next and new ones
 	uint32_t n_shadow_prev; // records made by the previous iteration, traced by this one's trace_kernel
+	uint32_t capacity;      // paths in flight at most (here, on the line begin_kernel reads anyway)
 	unsigned long long next_path;   // next path index to generate
 	unsigned long long total_paths;
 	unsigned long long rays_traced; // closest-hit rays (extension + camera)
@@ -243,6 +244,7 @@ struct RenderConsts
 {
 	uint64_t seed;
 	uint64_t first_global;   // global index of path 0
+	uint32_t max_bounces;
 };
 
 struct RenderState
@@ -437,7 +439,7 @@ private:
 	float render_pass(const RenderParams& params, double* film_device, const std::vector<BatchScene>* batch = nullptr);
 	struct Wave;
 	void ensure_capacity(uint32_t waves, uint32_t capacity, uint32_t grid);
-	void build_loop_graph(Wave& wave, const std::function<void(cudaGraphConditionalHandle)>& launches);
+	cudaGraphExec_t build_loop_graph(cudaStream_t stream, const std::function<void(cudaGraphConditionalHandle)>& launches);
 	// Coordinate descent over the launch shapes (pool depth, refill threshold, blocks per SM, and
 	// optionally leaf size), `measure` giving a candidate's calibration milliseconds; the winner is
 	// set on this scene.
@@ -455,18 +457,15 @@ private:
 	DeviceBuffer<float2>      m_env_alias;
 	DeviceScene               m_dev{};
 
-	uint32_t m_capacity = 0;   // path slots of each wave
-	uint32_t m_order_grid = 0;
 	LaunchConfig m_launch;
 	float m_max_origin_abs = 0.0f;
 	uint32_t m_bvh_builder = 0;
 	std::vector<uint32_t> m_material_types;   // per material (fingerprint)
 	uint32_t m_shade_kinds = 0;               // bit per shading kernel the materials need besides the matte one
-	// One of the wavefronts a render runs: its own part of the path pool, counters, stream and loop
-	// graph. Renders of many paths run two side by side (render_pass).
-	struct Wave
+	static constexpr uint32_t kMaxWaves = 2;
+	// A wavefront's part of the path pool.
+	struct WaveBuffers
 	{
-		cudaStream_t stream = nullptr;   // the first wave's is m_stream
 		DeviceSpan<uint32_t> path[2], meta[2];
 		DeviceSpan<float4>   thr[2], rad[2], prev[2], ro[2], rd[2];
 		DeviceSpan<uint2>    hits;
@@ -474,22 +473,39 @@ private:
 		DeviceSpan<float2>   sr[2];
 		DeviceSpan<uint32_t> sid[2];                // multi-scene renders: scene of each NEE record
 		DeviceSpan<uint32_t> req_single, req_mutual;
-		DeviceSpan<uint32_t> order;                 // shading order: kOrderLists lists of m_order_list slots
+		DeviceSpan<uint32_t> order;                 // shading order: kOrderLists lists of `order_list` slots
+	};
+	// The pool as renders of one number of wavefronts carve it (one such render runs at a time, so that
+	// the layouts lie on top of each other). A layout keeps the largest capacity asked of it, so that
+	// renders of other sizes use the same addresses, and the graphs that name them.
+	struct PoolLayout
+	{
+		uint32_t capacity = 0;     // path slots of each wave
+		uint32_t order_list = 0;
+		WaveBuffers buffers[kMaxWaves];
+	};
+	PoolLayout m_layouts[kMaxWaves];      // of renders of 1, 2 wavefronts
+	uint32_t m_order_grid = 0;            // the grid the class lists are laid out for
+	DeviceBuffer<unsigned char> m_pool;   // the layouts' one allocation (ensure_capacity)
+	// One of the wavefronts a render runs: its stream, counters and loop graphs. Renders of many paths run
+	// two side by side (render_pass).
+	struct LoopGraph
+	{
+		cudaGraphExec_t exec;
+		std::vector<uint64_t> key;   // everything its launches were given
+	};
+	struct Wave
+	{
+		cudaStream_t stream = nullptr;   // the first wave's is m_stream
 		DeviceBuffer<RenderState> state;
 		RenderState* host_state = nullptr;          // pinned staging of `state`
-		// the instantiated loop graph of the last render with everything its launches were given (kept
-		// across renders)
-		cudaGraphExec_t exec = nullptr;
-		std::vector<uint64_t> exec_key;
+		// the instantiated loop graphs of the last kKeptGraphs kinds of render, the last one first
+		std::vector<LoopGraph> graphs;
 	};
-	static constexpr uint32_t kMaxWaves = 2;
 	Wave m_waves[kMaxWaves];
-	DeviceBuffer<unsigned char> m_pool;   // the waves' buffers: one allocation, carved by ensure_capacity
-	uint32_t m_pool_waves = 0;
 	DeviceBuffer<float4>   m_samples; // 4 x 4 filters: radiance of every path of a pass
 	DeviceBuffer<uint32_t> m_inflight;   // previews: paths in flight per pixel
 	DeviceBuffer<BatchScene> m_batch_table;
-	uint32_t m_order_list = 0;
 
 	// learned guiding
 	GuideParams m_guide_params;
@@ -512,6 +528,7 @@ private:
 	cudaStream_t m_stream = nullptr;
 	cudaEvent_t m_events[2] = {nullptr, nullptr};   // a render's timing
 	uint64_t m_buffer_generation = 0;   // counts reallocations of buffers that a graph's launches name
+	uint64_t m_graph_generation = 0;    // the one that the kept loop graphs are of
 
 	unsigned long long m_last_rays = 0, m_last_shadow = 0, m_last_iterations = 0, m_last_launches = 0;
 	unsigned long long m_last_counts[4] = {0, 0, 0, 0};
