@@ -1,5 +1,6 @@
 // Render-scene entry points of the low-level C ABI (include/photon_gpu.h): a flat scene
 // description in, FP64 film sums and developed frames out.
+#include "pg_geometry.h"
 #include "pg_render_object.h"
 #include "scene_build.h"
 
@@ -233,6 +234,10 @@ int pgpu_scene_destroy(uint64_t id)
 		if(!render_registry().remove(id))
 		{
 			throw Error(PG_ERR_NOT_FOUND, "unknown scene id " + std::to_string(id));
+		}
+		if(render_registry().empty() && geometry_registry().empty())
+		{
+			trim_scratch();
 		}
 	});
 }

@@ -1,5 +1,6 @@
 #include "pg_runtime.h"
 
+#include <algorithm>
 #include <mutex>
 #include <set>
 #include <utility>
@@ -68,48 +69,76 @@ namespace
 {
 
 std::mutex g_scratch_mutex;
-cudaMemPool_t g_scratch_pools[kMaxDevices] = {};
-
-cudaMemPool_t scratch_pool()
+struct ScratchPool
 {
-	const int dev = current_device();
-	std::lock_guard<std::mutex> lock(g_scratch_mutex);
-	if(!g_scratch_pools[dev])
+	cudaMemPool_t pool = nullptr;
+	std::size_t live = 0;   // bytes of the buffers in use
+	std::size_t high = 0;   // the most that were in use since the pool was last cut back
+};
+ScratchPool g_scratch[kMaxDevices];
+
+// (the mutex is held)
+cudaMemPool_t make_scratch_pool(int dev)
+{
+	cudaMemPoolProps props{};
+	props.allocType = cudaMemAllocationTypePinned;
+	props.location.type = cudaMemLocationTypeDevice;
+	props.location.id = dev;
+	cudaMemPool_t pool = nullptr;
+	PG_CUDA_CHECK(cudaMemPoolCreate(&pool, &props));
+	uint64_t kept = kScratchKept;
+	const cudaError_t status = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &kept);
+	if(status != cudaSuccess)
 	{
-		cudaMemPoolProps props{};
-		props.allocType = cudaMemAllocationTypePinned;
-		props.location.type = cudaMemLocationTypeDevice;
-		props.location.id = dev;
-		cudaMemPool_t pool = nullptr;
-		PG_CUDA_CHECK(cudaMemPoolCreate(&pool, &props));
-		uint64_t kept = kScratchKept;
-		const cudaError_t status = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &kept);
-		if(status != cudaSuccess)
-		{
-			cudaMemPoolDestroy(pool);
-			cudaGetLastError();
-			throw Error(PG_ERR_CUDA, std::string("cudaMemPoolSetAttribute: ") + cudaGetErrorString(status));
-		}
-		g_scratch_pools[dev] = pool;
+		cudaMemPoolDestroy(pool);
+		cudaGetLastError();
+		throw Error(PG_ERR_CUDA, std::string("cudaMemPoolSetAttribute: ") + cudaGetErrorString(status));
 	}
-	return g_scratch_pools[dev];
+	return pool;
 }
 
 }// end anonymous namespace
 
 void* scratch_alloc(std::size_t bytes)
 {
+	const int dev = current_device();
+	ScratchPool& scratch = g_scratch[dev];
+	{
+		std::lock_guard<std::mutex> lock(g_scratch_mutex);
+		if(!scratch.pool)
+		{
+			scratch.pool = make_scratch_pool(dev);
+		}
+	}
 	void* p = nullptr;
-	PG_CUDA_CHECK(cudaMallocFromPoolAsync(&p, bytes, scratch_pool(), library_stream()));
+	PG_CUDA_CHECK(cudaMallocFromPoolAsync(&p, bytes, scratch.pool, library_stream()));
+	std::lock_guard<std::mutex> lock(g_scratch_mutex);
+	scratch.live += bytes;
+	scratch.high = std::max(scratch.high, scratch.live);
 	return p;
 }
 
-void scratch_free(void* p) noexcept
+void scratch_free(void* p, std::size_t bytes) noexcept
 {
-	// (the stream exists: the allocation was made on it)
+	// (device, pool and stream exist: the allocation was made from them)
 	try
 	{
-		cudaFreeAsync(p, library_stream());
+		cudaStream_t s = library_stream();
+		cudaFreeAsync(p, s);
+		ScratchPool& scratch = g_scratch[current_device()];
+		{
+			std::lock_guard<std::mutex> lock(g_scratch_mutex);
+			scratch.live -= bytes;
+			if(scratch.high <= kScratchKept || scratch.live > kScratchKept)
+			{
+				return;
+			}
+			scratch.high = scratch.live;
+		}
+		// The release threshold acts at a synchronize only, and a call's last one is before its buffers are freed:
+		// what a large call took beyond the threshold would stay until somebody synchronizes again.
+		cudaStreamSynchronize(s);
+		cudaMemPoolTrimTo(scratch.pool, kScratchKept);
 	}
 	catch(...)
 	{
@@ -118,14 +147,33 @@ void scratch_free(void* p) noexcept
 
 void trim_scratch()
 {
-	std::lock_guard<std::mutex> lock(g_scratch_mutex);
-	for(cudaMemPool_t pool : g_scratch_pools)
+	const int dev = current_device();
+	if(g_scratch[dev].pool)
 	{
-		if(pool)
+		cudaStreamSynchronize(library_stream());   // buffers count as freed once the host has seen the stream pass them
+	}
+	std::lock_guard<std::mutex> lock(g_scratch_mutex);
+	for(const ScratchPool& scratch : g_scratch)
+	{
+		if(scratch.pool)
 		{
-			cudaMemPoolTrimTo(pool, 0);
+			cudaMemPoolTrimTo(scratch.pool, 0);
 		}
 	}
+}
+
+void* device_alloc(std::size_t bytes)
+{
+	void* p = nullptr;
+	cudaError_t status = cudaMalloc(&p, bytes);
+	if(status == cudaErrorMemoryAllocation)
+	{
+		(void)cudaGetLastError();
+		trim_scratch();
+		status = cudaMalloc(&p, bytes);
+	}
+	PG_CUDA_CHECK(status);
+	return p;
 }
 
 unsigned char* pinned_stage()

@@ -146,6 +146,9 @@ private:
 	cudaEvent_t m_event = nullptr;
 };
 
+// cudaMalloc; out of memory, the scratch pool's kept bytes go back first.
+void* device_alloc(std::size_t bytes);
+
 // Device buffer with RAII ownership.
 template<typename T>
 class DeviceBuffer
@@ -177,7 +180,7 @@ public:
 		release();
 		if(n > 0)
 		{
-			PG_CUDA_CHECK(cudaMalloc(reinterpret_cast<void**>(&m_ptr), n * sizeof(T)));
+			m_ptr = static_cast<T*>(device_alloc(n * sizeof(T)));
 		}
 		m_size = n;
 	}
@@ -218,12 +221,14 @@ private:
 
 // Device memory for one call, in stream order on the library stream: taken from the device's scratch
 // pool and handed back when the buffer's scope ends, after the work queued by then. cudaMalloc and
-// cudaFree, which wait for the device, cost a query of 1,000 rays more than its kernels. The pool
-// keeps at most kScratchKept bytes between calls (trim_scratch gives those back too) and may be
-// used from several threads.
-constexpr std::size_t kScratchKept = std::size_t(256) << 20;
+// cudaFree, which wait for the device, cost a query of 1,000 rays more than its kernels. The pool may be
+// used from several threads. Between calls it keeps at most kScratchKept bytes (0.3 % of the device's
+// memory; the largest batches of the guiding network that are ordinary take 310 MiB): a call that took
+// more gives the rest back when its buffers go. The kept bytes go back with the last geometry or scene,
+// and when an allocation outside the pool finds no room (device_alloc).
+constexpr std::size_t kScratchKept = std::size_t(512) << 20;
 void* scratch_alloc(std::size_t bytes);
-void scratch_free(void* p) noexcept;
+void scratch_free(void* p, std::size_t bytes) noexcept;
 void trim_scratch();
 
 template<typename T>
@@ -231,7 +236,7 @@ class ScratchBuffer
 {
 public:
 	explicit ScratchBuffer(std::size_t n) : m_ptr(n ? static_cast<T*>(scratch_alloc(n * sizeof(T))) : nullptr), m_size(n) {}
-	~ScratchBuffer() { if(m_ptr) { scratch_free(m_ptr); } }
+	~ScratchBuffer() { if(m_ptr) { scratch_free(m_ptr, bytes()); } }
 	ScratchBuffer(const ScratchBuffer&) = delete;
 	ScratchBuffer& operator = (const ScratchBuffer&) = delete;
 	T* get() const { return m_ptr; }
