@@ -3085,14 +3085,7 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 			throw Error(PG_ERR_CUDA, "render: guiding network kernel timed out waiting on its tensor cores");
 		}
 	}
-	if(final_counters.error & PG_DEV_ERR_STACK)
-	{
-		throw Error(PG_ERR_STACK_OVERFLOW, "render: BVH traversal stack overflow");
-	}
-	if(!done)
-	{
-		throw Error(PG_ERR_ITERATION_LIMIT, "render: iteration limit reached before all paths finished");
-	}
+	check_render_end(final_counters.error, done);
 	return ms;
 }
 

@@ -205,6 +205,22 @@ void require_same_device(int owner_device, const char* what)
 	check_same_device(owner_device, current_device(), what);
 }
 
+void check_render_end(uint32_t device_errors, bool done)
+{
+	if(device_errors & PG_DEV_ERR_STACK)
+	{
+		throw Error(PG_ERR_STACK_OVERFLOW, "render: BVH traversal stack overflow");
+	}
+	if(device_errors & PG_DEV_ERR_QUEUE)
+	{
+		throw Error(PG_ERR_QUEUE_OVERFLOW, "render: the queues ran empty before all paths finished");
+	}
+	if(!done)
+	{
+		throw Error(PG_ERR_ITERATION_LIMIT, "render: iteration limit reached before all paths finished");
+	}
+}
+
 void allow_shared_memory(const void* kernel, int bytes)
 {
 	static std::mutex mutex;

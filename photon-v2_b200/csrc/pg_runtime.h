@@ -257,6 +257,9 @@ unsigned char* pinned_stage();
 // asked for, once per kernel and device).
 void allow_shared_memory(const void* kernel, int bytes);
 
+// Throws what a render's device error flags (DeviceErrorFlag), or its end before the last path, say.
+void check_render_end(uint32_t device_errors, bool done);
+
 // Number of SMs of the current device (grid sizing).
 int sm_count();
 
