@@ -133,7 +133,8 @@ extern PH_API void phGpuClearFilm(PhUInt64 engineId);
 extern PH_API void phGpuGetRenderInfo(PhUInt64 engineId, PhFloat64* out_deviceMs, PhUInt64* out_paths,
                                       PhUInt64* out_rays, PhUInt64* out_shadowRays, PhFloat64* out_updateSeconds);
 
-/* Kernel launches of the last phRender (three to nine per wavefront iteration). */
+/* Kernel launches of the last phRender: three to ten per wavefront iteration, one per two of them (four when
+ * the guiding network trains) that ends or continues the loop, a training step's six to eight, and the film's. */
 extern PH_API PhUInt64 phGpuGetLaunchCount(PhUInt64 engineId);
 /* Profiling render of `samplesPerPixel` samples into a scratch film (the engine's own image is
  * untouched). mode 1: plain launches with CUDA events around every kernel; mode 2: traversal

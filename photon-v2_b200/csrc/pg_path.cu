@@ -2518,8 +2518,8 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 	// Two wavefronts, each with half of the paths and of the pool, run side by side on streams of their
 	// own: a traversal launch ends with a tail of its longest rays (a fifth of its time on the bench
 	// scene), in which the other wavefront's kernels take over the SMs that have run dry. That pays
-	// where the paths fill the pool at least twice (Cornell box at 64 samples 4.82 to 4.45 ms, bench scene
-	// at 16 samples 18.4 to 18.0 ms, 8 scenes in one wavefront 104.6 to 101.9 ms); below, the queues only
+	// where the paths fill the pool at least twice (Cornell box at 64 samples 4.82 to 4.52 ms, bench scene
+	// at 16 samples 18.3 to 18.1 ms, 8 scenes in one wavefront 105.0 to 102.2 ms); below, the queues only
 	// drain, a half-empty launch takes as long as a full one, and one wavefront is better (slit room at
 	// 2 samples, which fill the pool once, 14.55 against 14.84 ms). Guided renders share a training
 	// batch and profiled ones time kernel by kernel: one wavefront.
@@ -2665,7 +2665,10 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 	}
 	// Where the matte kernel takes every slot and none is guided, shading in slot order saves the
 	// classification and reads the path state coalesced; the misses and light hits that it leaves among
-	// the matte vertices end early (the Cornell box at 64 samples: 5.00 to 4.76 ms).
+	// the matte vertices end early (the Cornell box at 64 samples: 5.00 to 4.76 ms; a matte city of 0.4 M
+	// triangles 9.19 to 9.02, a matte slit room 8.72 to 8.49). Where half of the rays miss and look the dome
+	// up, the classes are the faster way (a matte sphere of 1.3 M triangles under a dome 16.7 against
+	// 17.8 ms, without the dome 16.5 against 16.8).
 	const bool classify = kinds != 0u || guided;
 	// The NEE segments made by an iteration's shading are traced by the next iteration's
 	// trace_kernel together with its closest-hit rays (one launch, one tail). Training runs in
@@ -2887,10 +2890,10 @@ float RenderScene::render_pass(const RenderParams& params, double* film_sums, co
 	if(params.mode == PG_RENDER_GRAPH)
 	{
 		// One graph = a loop on the device over periods (two iterations, ping -> pong -> ping; four when
-		// training): the last kernel of a period decides whether another follows, so that no
-		// iteration runs after the last path and the host only waits. (Periods launched by the host
-		// in batches of 4, 8, ... ran up to 14 empty iterations on short renders: a 64 x 48 thumbnail
-		// took 24 iterations for its 9.) Building a graph takes about 270 us, more than a thumbnail's whole
+		// training): the last kernel of a period decides whether another follows, so that at
+		// most the rest of a period (one iteration, three when training) runs after the last path and the
+		// host only waits. (Periods launched by the host in batches of 4, 8, ... ran up to 14 empty
+		// iterations on short renders: a 64 x 48 thumbnail took 24 iterations for its 9, now 10.) Building a graph takes about 270 us, more than a thumbnail's whole
 		// render, so a wave keeps those of the last kinds of render, and what changes from call to
 		// call (samples, depth, seed, pool share) reaches the kernels through device memory.
 		if(m_graph_generation != m_buffer_generation)

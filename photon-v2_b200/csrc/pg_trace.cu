@@ -50,7 +50,7 @@ constexpr int kTraceBlock = kTraversalBlock;
 constexpr int kTraceMinBlocks = 8;
 // Rays of several scenes carry their tree's two addresses, which do not fit 64 registers (100 bytes of
 // spills): 72 registers at seven blocks. Eight scenes at 1/8 of their samples in one wavefront: 102.0 ms
-// a call with eight blocks, 98.2 with seven, 104.3 with six.
+// a call with eight blocks, 97.8 with seven, 104.3 with six.
 constexpr int kTraceMinBlocksMulti = 7;
 
 struct HitRecord

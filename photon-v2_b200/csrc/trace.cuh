@@ -224,8 +224,9 @@ __device__ __forceinline__ float2 planes(uint32_t near_word, uint32_t far_word, 
 // Intersects the 8 child boxes of a wide node. Returns the hit mask: bits 24..31 are internal
 // children at key (slot ^ oct), bits 0..23 are leaf triangles relative to tri_base.
 //
-// The traversal loop is bound by instruction issue (70 % of the slots) with the byte-to-float
-// conversions close behind (66 % of their pipe), so the test spends as few of both as it can: an
+// The traversal loop was bound by instruction issue (70 % of the slots) with the byte-to-float
+// conversions close behind (62 % of their pipe), so the test spends as few of both as it can (now 61 to
+// 69 % and 43 to 54 % in a render's first three iterations): an
 // axis's near and far plane go through one paired FMA, the meta bytes of four children are decoded
 // together, and the three planes of a side meet in one three-input minimum or maximum. One million
 // rays against 2 M triangles: 560 M to 496 M warp instructions, 734 us to 681 us. Taking half or all
